@@ -270,19 +270,25 @@ MOMED_API int  momed_serve_stop(momed_server* s);
 MOMED_API int  momed_block_tuning(momed_handle* h, int32_t nb, int32_t precision, int32_t has_param,
                                   int32_t* rows_per_warp, int32_t* grid_mult, double* ms, double* ms_default);
 
-/* Hit cache of the matrix-free map: for the current sector basis and term list, the target row
- * and term slot of every off-diagonal (row, term) hit (8 bytes each) and each row's diagonal
- * sums, so that a map skips the candidate stage (mask tests, signs, index lookups) and forms
- * only the values, from the term list, at each application.  The eigensolvers build it at their
- * start when it fits a quarter of the free device memory and no HBM budget is set; when it does
- * not, its slot mode (the term slot of each hit only, 2 bytes, for at most 65536 terms; the
- * single-vector map then forms each target itself) when that fits 30% (MOMED_HITCACHE=0: never,
- * =1: full whatever its size, =2: slot mode); momed_build_hit_cache builds it on request (the
- * slot mode under MOMED_HITCACHE=2; MOMED_ENOMEM when it does not fit, MOMED_ESTATE while a
- * sparse matrix is built).  It is
- * dropped with the basis, the operator, a sparse-matrix build, or new amplitudes of a
- * parametrised operator.  No reference counterpart: the reference map evaluates every term at
- * every application (ka_linearmap_kernel!, MomentumED/src/method/gpu_interface.jl:128-163). */
+/* Hit cache of the matrix-free map: what a map computes again at every application, kept for the
+ * current sector basis and term list; only the values are formed from the term list at each
+ * application (a new u needs no rebuild).  A full cache holds, for single-vector maps of operators
+ * whose off-diagonal terms are all two-body, the tables of the pair-factorised product (sectors of
+ * at least 2^20 (row, pair) entries with enough free pairs per state; MOMED_PAIRMAP=0: never, =1:
+ * whatever the size), and otherwise, and from the first block map on, the target row and term slot
+ * of every off-diagonal (row, term) hit (8 bytes each) with each row's diagonal sums.  The
+ * eigensolvers build it at their start when it fits a quarter of the free device memory and no HBM
+ * budget is set; when it does not, its slot mode (the term slot of each hit only, 2 bytes, for at
+ * most 65536 terms; the single-vector map then forms each target itself) when that fits 30%
+ * (MOMED_HITCACHE=0: never, =1: full whatever its size, =2: slot mode); momed_build_hit_cache builds
+ * it on request (the slot mode under MOMED_HITCACHE=2; MOMED_ENOMEM when it does not fit,
+ * MOMED_ESTATE while a sparse matrix is built).  hits counts the off-diagonal hits; bytes is the
+ * device memory of the cache, the records of later block maps included.  momed_matvec builds the
+ * pair tables by itself at the second call on a basis and operator (same memory rule; not reported
+ * as a hit cache).  The cache is dropped with the basis, the operator, a sparse-matrix build, or
+ * new amplitudes of a parametrised operator.  No reference counterpart: the reference map evaluates
+ * every term at every application (ka_linearmap_kernel!,
+ * MomentumED/src/method/gpu_interface.jl:128-163). */
 MOMED_API int  momed_build_hit_cache(momed_handle* h, int64_t* hits, int64_t* bytes);
 MOMED_API int  momed_hit_cache_info(momed_handle* h, int32_t* built, int64_t* hits, int64_t* bytes,
                                     double* build_ms);          /* built: 0 none, 1 full, 2 slot mode */

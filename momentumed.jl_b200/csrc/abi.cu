@@ -172,6 +172,9 @@ void upload_operator(momed_handle* h, const double* amp_a, const double* amp_b, 
         up(op.ampb32, B32);
     }
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+    h->op.h_in = std::move(t_in);
+    h->op.h_out = std::move(t_out);
+    h->pplan.state = -1;
     h->op_order = std::move(ord);
     h->recipe.set = false;                 // a recipe describes the operator it was attached to
     h->op_mask_or = mask_or;
@@ -181,9 +184,8 @@ void upload_operator(momed_handle* h, const double* amp_a, const double* amp_b, 
     h->hcache.release();
 }
 
-// Build the index when the basis changed or the operator reaches bits outside it, and
-// validate the operator once: zero targets outside the basis enables the unchecked lookup.
-void ensure_ready(momed_handle* h) {
+// Build the index when the basis changed or the operator reaches bits outside it.
+void ensure_index(momed_handle* h) {
     MOMED_REQUIRE(!h->sparse_only, MOMED_ESTATE,
                   "the handle holds an uploaded matrix without a basis (momed_set_sparse_csr); set a basis first");
     MOMED_REQUIRE(h->n > 0, MOMED_ESTATE, "set a basis first (momed_set_basis / momed_select_sector)");
@@ -194,6 +196,12 @@ void ensure_ready(momed_handle* h) {
         h->index_dirty = false;
         h->op_validated = false;
     }
+}
+
+// The index, and the operator validated once: zero targets outside the basis enables the
+// unchecked lookup of the candidate kernels.  (The pair tables compare keys as they are built.)
+void ensure_ready(momed_handle* h) {
+    ensure_index(h);
     if (!h->op_validated) {
         if (h->index.mode != INDEX_SEARCH) {
             h->index.mode = INDEX_CHECKED;
@@ -516,7 +524,16 @@ int momed_matvec(momed_handle* h, const void* x, void* y, int32_t precision, int
     return guarded(h, [&]() {
         MOMED_REQUIRE(x && y, MOMED_EINVAL, "null vector");
         MOMED_REQUIRE(precision == MOMED_C128 || precision == MOMED_C64, MOMED_EINVAL, "unknown precision");
-        if (!h->sparse.built) ensure_ready(h);
+        if (!h->sparse.built) {
+            ensure_index(h);
+            if (!h->hcache.built && !h->hcache.pair.built) {
+                // a map applied again and again (an outer Krylov code): from the second call on a
+                // basis and operator, the pair tables, when they are admitted as the solvers' are
+                if (h->hcache.plain_calls > 0) ensure_plain_pair(h);
+                else ++h->hcache.plain_calls;
+            }
+            if (!h->hcache.built && !h->hcache.pair.built) ensure_ready(h);
+        }
         const int64_t n = h->n;
         cudaStream_t st = h->stream;
         const size_t es = precision == MOMED_C128 ? 16 : 8;
@@ -532,6 +549,10 @@ int momed_matvec(momed_handle* h, const void* x, void* y, int32_t precision, int
             launch_spmv_c128(h->sparse, (const double2*)dx, (double2*)dy, n, st);
         else if (h->sparse.built)
             launch_spmv_c64(h->sparse, (const float2*)dx, (float2*)dy, n, st);
+        else if (h->hcache.pair.built && precision == MOMED_C128)
+            launch_pair_c128(h, (const double2*)dx, (double2*)dy, h->u, st);
+        else if (h->hcache.pair.built)
+            launch_pair_c64(h, (const float2*)dx, (float2*)dy, h->u, st);
         else if (h->hcache.built && precision == MOMED_C128)
             launch_matvec_hc_c128(h, (const double2*)dx, (double2*)dy, h->op.has_b ? h->u_dev.p : nullptr, n, st);
         else if (h->hcache.built)
@@ -725,7 +746,7 @@ int momed_build_hit_cache(momed_handle* h, int64_t* hits, int64_t* bytes) {
     return guarded(h, [&]() {
         MOMED_REQUIRE(!h->sparse.built && !h->sparse_only, MOMED_ESTATE,
                       "a sparse matrix is built: maps read it (momed_release_sparse first)");
-        ensure_ready(h);
+        ensure_index(h);
         const char* e = std::getenv("MOMED_HITCACHE");
         build_hit_cache(h, (e && e[0] == '2') ? 2 : 1);     // MOMED_HITCACHE=2: the slot mode
         if (hits) *hits = h->hcache.nnz;

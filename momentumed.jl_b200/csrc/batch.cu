@@ -384,11 +384,17 @@ int sms() {
 
 template <typename VT> struct BlockMv;
 template <> struct BlockMv<float2> {
-    static void run(momed_handle* h, const float2* x, float2* y, const float* u, int nb) {
+    // u0: the host's copy of u[0]; one right-hand side runs the single-vector map over the pair tables
+    static void run(momed_handle* h, const float2* x, float2* y, const float* u, int nb, double u0) {
         prof_begin(h);
         if (h->sparse.built) {   // the sparse method's entries (momed_build_sparse)
             launch_block_spmv_c64(h->sparse, x, y, h->op.has_b ? u : nullptr, nb, h->n, h->stream);
             prof_end(h, MOMED_KERNEL_BLOCK_SPMV_C64);
+            return;
+        }
+        if (nb == 1 && h->hcache.pair.built) {
+            launch_pair_c64(h, x, y, u0, h->stream);
+            prof_end(h, MOMED_KERNEL_HC_BLOCK_C64);
             return;
         }
         if (h->hcache.full()) {
@@ -401,8 +407,13 @@ template <> struct BlockMv<float2> {
     }
 };
 template <> struct BlockMv<double2> {
-    static void run(momed_handle* h, const double2* x, double2* y, const double* u, int nb) {
+    static void run(momed_handle* h, const double2* x, double2* y, const double* u, int nb, double u0) {
         prof_begin(h);
+        if (nb == 1 && h->hcache.pair.built) {
+            launch_pair_c128(h, x, y, u0, h->stream);
+            prof_end(h, MOMED_KERNEL_HC_BLOCK_C128);
+            return;
+        }
         if (h->hcache.full()) {
             launch_block_hc_c128(h, x, y, u, nb, h->n, h->stream);
             prof_end(h, MOMED_KERNEL_HC_BLOCK_C128);
@@ -428,6 +439,7 @@ struct BlockLanczos {
     DevBuf<int> flag, any;
     DevBuf<RT> ud;
     int64_t launches = 0;
+    double u0;           // u of the first right-hand side
     double dgks = 0.5;   // second Gram-Schmidt pass when |w'|^2 < dgks |w|^2 (set by run)
     // The steps of a restart cycle (k .. m-1) as one CUDA graph: captured the first time a cycle
     // starts at k on a given basis buffer (the restart alternates two), replayed afterwards.  A
@@ -487,7 +499,7 @@ struct BlockLanczos {
         for (int j = k; j < m; ++j) step(j);
     }
 
-    BlockLanczos(momed_handle* hh, int mm, const std::vector<double>& u) : h(hh), N(hh->n), m(mm), st(hh->stream) {
+    BlockLanczos(momed_handle* hh, int mm, const std::vector<double>& u) : h(hh), N(hh->n), m(mm), st(hh->stream), u0(u[0]) {
         {
             const char* e = std::getenv("MOMED_GRAPHS");
             use_graphs = !(e && e[0] == '0') && !hh->prof;   // per-launch timing needs eager launches
@@ -573,7 +585,7 @@ struct BlockLanczos {
     }
     void step(int j) {
         VT* w = col(j + 1);
-        BlockMv<VT>::run(h, col(j), w, ud.p, NB);   // counted by its launcher
+        BlockMv<VT>::run(h, col(j), w, ud.p, NB, u0);   // counted by its launcher
         const int nc = j + 1;
         proj(nc, w, coefA.p, nullptr);
         update(nc, coefA.p, w, nullptr, nullptr);
@@ -1072,7 +1084,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
         MOMED_CUDA_TRY(cudaMemcpyAsync(ud64.p, uh.data(), NB * sizeof(double), cudaMemcpyHostToDevice, st));
         MOMED_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    for (int i = 0; i < k1; ++i) BlockMv<double2>::run(h, Xb.p + (size_t)i * stride, Wb.p + (size_t)i * stride, ud64.p, NB);
+    for (int i = 0; i < k1; ++i) BlockMv<double2>::run(h, Xb.p + (size_t)i * stride, Wb.p + (size_t)i * stride, ud64.p, NB, uv[0]);
     matvecs += (int64_t)k1 * nu;
     matvecs64 += (int64_t)k1 * nu;
     std::vector<std::vector<double>> th(NB, std::vector<double>(k1, 0.0));
@@ -1433,7 +1445,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                 // their residuals; the other anchors enter only through the Ritz values' gaps and
                 // keep W' from the Lanczos relation), exact residuals, final acceptance
                 for (int i = 0; i < nev; ++i)
-                    BlockMv<double2>::run(h, Xb.p + (size_t)i * stride, Wb.p + (size_t)i * stride, ud64.p, NB);
+                    BlockMv<double2>::run(h, Xb.p + (size_t)i * stride, Wb.p + (size_t)i * stride, ud64.p, NB, uv[0]);
                 matvecs += (int64_t)nev * nu;
                 matvecs64 += (int64_t)nev * nu;
                 residuals();
@@ -1466,7 +1478,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
         broken3 = r3.broken;
         // FP64 residuals of the phase-3 pairs
         for (int i = 0; i < nev; ++i)
-            BlockMv<double2>::run(h, X3.p + (size_t)i * stride, Wb.p + (size_t)i * stride, ud64.p, NB);
+            BlockMv<double2>::run(h, X3.p + (size_t)i * stride, Wb.p + (size_t)i * stride, ud64.p, NB, uv[0]);
         matvecs += (int64_t)nev * nu;
         matvecs64 += (int64_t)nev * nu;
         const int rg = std::max(1, std::min<int>((int)((stride + 255) / 256), 512));
@@ -1561,12 +1573,16 @@ using namespace momed;
 
 int momed_batch_solve_impl(momed_handle* h, const momed_solve_opts* o, const double* u, int32_t nu, double* vals,
                            double* resid, double* vecs, momed_info* info) {
-    ensure_ready(h);
-    if (!h->sparse.built) ensure_hit_cache(h);
     // without a second operator (momed_set_scatter) every parameter solves H = A
     MOMED_REQUIRE(nu >= 1 && nu <= 32, MOMED_EINVAL, "nu must be 1..32 per call");
     int nb = 1;
     while (nb < nu) nb <<= 1;
+    ensure_index(h);
+    if (!h->sparse.built) {
+        if (nb == 1) ensure_hit_cache(h);
+        else ensure_hit_records(h);
+    }
+    if (nb > 1 || !h->hcache.pair.built) ensure_ready(h);
     switch (nb) {
         case 1: return run_batch<1>(h, o, u, nu, vals, resid, vecs, info);
         case 2: return run_batch<2>(h, o, u, nu, vals, resid, vecs, info);

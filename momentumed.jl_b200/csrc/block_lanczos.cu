@@ -833,6 +833,8 @@ int block_size_for(momed_handle* h, int nev, int precision) {
     // Mixed precision goes to the batched solver with one right-hand side instead (its anchored
     // FP64 refinement): two-component 4x6, nev 8: 2.73 s against 7.56 s for the mixed block solver
     // (whose FP64 phase restarts from B of the refined vectors) and 4.2 s for the FP64 one.
+    // The pair tables' single-vector map has no gather for the block to share.
+    if (h->hcache.pair.built && !h->hcache.records) return 0;
     if (nev < 6 || h->n < (h->hcache.full() ? 2000000 : 500000)) return 0;
     if (precision == MOMED_PREC_MIXED) return 0;
     return nev <= 10 ? 4 : 8;
@@ -844,6 +846,8 @@ int block_size_for(momed_handle* h, int nev, int precision) {
 bool eigsolve_block(momed_handle* h, const momed_solve_opts* o, int nev, int B, const double2* start64, double2* X,
                     std::vector<double>& theta, std::vector<double>& res, int& nconv, int& restarts, int64_t& matvecs,
                     int64_t& matvecs64) {
+    ensure_ready(h);
+    ensure_hit_records(h);
     try {
         switch (B) {
             case 4: solve_blocked<4>(h, o, nev, start64, X, theta, res, nconv, restarts, matvecs, matvecs64); break;

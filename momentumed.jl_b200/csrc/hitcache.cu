@@ -17,15 +17,17 @@
 //   diag[2n]               the row's diagonal terms summed, A part and B part (FP64, and c64)
 //
 // 8 bytes per hit, against 20-44 for a stored matrix entry; the values are still formed from the
-// term list at every application, so a new u needs no rebuild.  A map over the cache reads the
+// term list at every application, so a new u needs no rebuild.  A map over the records reads the
 // hit stream (coalesced), the amplitude of each hit's term slot (the term list stays in L1/L2)
-// and gathers x.  The cache is built when it fits a quarter of the free HBM (MOMED_HITCACHE=0
-// turns it off, =1 builds it whatever its size); sectors whose hits do not fit (the 35M-state
-// 4x9 sectors: ~170 GB) get the slot mode instead: per hit only its term slot (uint16, 2 bytes;
-// 43 GB for a 4x9 Ne = 12 sector), from which the single-vector map forms the target exactly as
-// the candidate map does (mask arithmetic, sign, two table reads) without the candidate stage;
-// the block maps read full caches only.  It is dropped with the basis, the operator or the
-// amplitudes (a twisted-boundary update) it was built from.
+// and gathers x.  Block maps run over the records; a single-vector map runs over them where the
+// operator or the sector does not take the pair form (pairmap.cu), which a full cache prefers.  The
+// cache is built when it fits a quarter of the free HBM (MOMED_HITCACHE=0 turns it off, =1 builds
+// it whatever its size); sectors whose tables do not fit (the 35M-state 4x9 sectors: ~170 GB of
+// records) get the slot mode instead: per hit only its term slot (uint16, 2 bytes; 43 GB for a 4x9
+// Ne = 12 sector), from which the single-vector map forms the target exactly as the candidate map
+// does (mask arithmetic, sign, two table reads) without the candidate stage; the block maps read
+// records only.  It is dropped with the basis, the operator or the amplitudes (a twisted-boundary
+// update) it was built from.
 #include <chrono>
 #include <cstdlib>
 #include <string>
@@ -33,6 +35,8 @@
 #include "blockio.cuh"
 
 namespace momed {
+
+void ensure_ready(momed_handle* h);
 
 namespace {
 
@@ -558,27 +562,61 @@ int64_t slot_cache_bytes(int64_t n, int64_t hits) {
     return (n + 1) * 8 + n * (32 + 16) + hits * 2;
 }
 
-// The full cache when it fits a quarter of the free memory, else the slot mode when that fits
-// 30% (term slots must fit 16 bits); MOMED_HITCACHE=0: none, =1: full whatever its size, =2:
-// slot mode whatever its size.
-int hit_cache_wanted(const momed_handle* h) {
+// 0: no cache; 1: full whatever its size (MOMED_HITCACHE=1); 2: slot mode whatever its size (=2);
+// -1: by size
+static int cache_policy(const momed_handle* h) {
     const char* e = std::getenv("MOMED_HITCACHE");
     if (e && e[0] == '0') return 0;
     if (!h->hit_cache_ok || h->hbm_budget > 0 || h->sparse.built || h->sparse_only || h->n <= 0 || !h->op_set)
         return 0;
-    const bool slots_ok = h->op.nterms <= 65536;
     if (e && e[0] == '1') return 1;
-    if (e && e[0] == '2') return slots_ok ? 2 : 0;
+    if (e && e[0] == '2') return 2;
+    return -1;
+}
+
+static double free_bytes() {
     size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
-    if ((double)hit_cache_bytes(h->n, h->nnz) <= 0.25 * (double)free_b) return 1;
-    if (slots_ok && (double)slot_cache_bytes(h->n, h->nnz) <= 0.30 * (double)free_b) return 2;
+    return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess ? (double)free_b : 0.0;
+}
+
+// Hit records when they fit a quarter of the free memory, else the slot mode when that fits 30%
+// (term slots must fit 16 bits); the operator has been validated (h->nnz).
+int hit_cache_wanted(const momed_handle* h) {
+    const bool slots_ok = h->op.nterms <= 65536;
+    const int pol = cache_policy(h);
+    if (pol == 2) return slots_ok ? 2 : 0;
+    if (pol >= 0) return pol;
+    const double fb = free_bytes();
+    if ((double)hit_cache_bytes(h->n, h->nnz) <= 0.25 * fb) return 1;
+    if (slots_ok && (double)slot_cache_bytes(h->n, h->nnz) <= 0.30 * fb) return 2;
     return 0;
 }
 
-void build_hit_cache(momed_handle* h, int mode) {
+// Device memory a full cache will hold: the pair tables for single-vector maps where the operator
+// takes that form, else (and for block maps) the hit records.  Needs h->nnz for the records.
+int64_t full_cache_bytes(momed_handle* h, bool block_maps) {
+    if (!block_maps && pair_possible(h)) return pair_bytes(h);
+    return hit_cache_bytes(h->n, h->nnz);
+}
+
+// The pair tables as a full cache (no hit records yet).  False: declined.
+static bool build_pair_cache(momed_handle* h) {
     HitCache& hc = h->hcache;
-    hc.release();
+    const auto t0 = std::chrono::steady_clock::now();
+    if (!hc.pair.built && !build_pair_map(h)) return false;
+    if (hc.built) return true;                  // beside records built before
+    hc.mode = 1;
+    hc.nnz = hc.pair.hits;
+    hc.bytes = hc.pair.bytes + hit_cache_bytes(h->n, hc.nnz);   // with the records of later block maps
+    hc.build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    hc.built = true;
+    return true;
+}
+
+// hit records (mode 1) or slots (mode 2) of every off-diagonal hit; pair tables stay
+static void build_records(momed_handle* h, int mode) {
+    HitCache& hc = h->hcache;
+    ensure_ready(h);
     MOMED_REQUIRE(mode == 1 || mode == 2, MOMED_EINVAL, "hit cache: unknown mode");
     MOMED_REQUIRE(mode == 1 || h->op.nterms <= 65536, MOMED_EINVAL, "hit cache: slot mode needs <= 65536 terms");
     const auto t0 = std::chrono::steady_clock::now();
@@ -641,23 +679,84 @@ void build_hit_cache(momed_handle* h, int mode) {
         throw Error{MOMED_EINVAL, "hit cache: count and fill passes disagree on " + std::to_string(bad) + " hits"};
     }
     hc.nnz = nnz;
-    hc.bytes = need;
+    hc.bytes = need + (hc.pair.built ? hc.pair.bytes : 0);
     hc.mode = mode;
+    hc.records = mode == 1;
     hc.build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     hc.built = true;
 }
 
+void build_hit_cache(momed_handle* h, int mode) {
+    HitCache& hc = h->hcache;
+    hc.release();
+    if (mode == 1 && pair_possible(h) && (double)pair_bytes(h) <= 0.9 * free_bytes() && build_pair_cache(h)) return;
+    build_records(h, mode);
+}
+
+void build_hit_records(momed_handle* h) {
+    if (!h->hcache.records) build_records(h, 1);
+}
+
 // The automatic build is an optimisation: when its allocations are refused (memory taken by
 // another handle between the size check and the build) the solve goes on over the candidate map.
+// Single-vector maps: the pair tables when they fit a quarter of the free memory, else the records.
 void ensure_hit_cache(momed_handle* h) {
-    if (h->hcache.built) return;
+    HitCache& hc = h->hcache;
+    const int pol = cache_policy(h);
+    if (hc.pair.built && !hc.built && pol) {      // built for momed_matvec: it serves the solver too
+        build_pair_cache(h);
+        return;
+    }
+    if (pol && pol != 2 && !hc.pair.built && !(hc.built && hc.mode == 2) && pair_possible(h) &&
+        (pol == 1 || (double)pair_bytes(h) <= 0.25 * free_bytes())) {
+        try {
+            build_pair_cache(h);
+        } catch (const Error& e) {
+            if (e.code != MOMED_ENOMEM) throw;
+            hc.pair.release();
+        }
+    }
+    if (hc.built || !pol) return;
+    ensure_ready(h);
     const int mode = hit_cache_wanted(h);
     if (!mode) return;
     try {
-        build_hit_cache(h, mode);
+        build_records(h, mode);
     } catch (const Error& e) {
         if (e.code != MOMED_ENOMEM) throw;
-        h->hcache.release();
+        hc.release();
+    }
+}
+
+// Block maps: the hit records by the same rule (beside pair tables if a full cache was asked for).
+void ensure_hit_records(momed_handle* h) {
+    HitCache& hc = h->hcache;
+    if (hc.records || (hc.built && hc.mode == 2) || (!hc.built && !cache_policy(h))) return;
+    ensure_ready(h);
+    int mode = 1;
+    if (!hc.built) mode = hit_cache_wanted(h);
+    else if ((double)hit_cache_bytes(h->n, hc.nnz) > (cache_policy(h) == 1 ? 0.9 : 0.25) * free_bytes()) mode = 0;
+    if (!mode) return;
+    try {
+        build_records(h, mode);
+    } catch (const Error& e) {
+        if (e.code != MOMED_ENOMEM) throw;
+        if (!hc.pair.built) hc.release();
+        else hc.release_records();
+    }
+}
+
+// momed_matvec without a cache: the pair tables alone, under the automatic rule (not reported as a
+// hit cache, which the caller did not ask for).
+void ensure_plain_pair(momed_handle* h) {
+    HitCache& hc = h->hcache;
+    if (cache_policy(h) != -1 || !pair_possible(h) || (double)pair_bytes(h) > 0.25 * free_bytes()) return;
+    try {
+        build_pair_map(h);
+    } catch (const Error& e) {
+        if (e.code != MOMED_ENOMEM) throw;
+        hc.pair.release();
+        hc.plain_calls = 0;
     }
 }
 
@@ -728,7 +827,7 @@ template <typename R>
 static void block_hc_dispatch(const momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* y, const R* u,
                               int32_t nb, int64_t rows, cudaStream_t st) {
     if (rows <= 0) return;
-    MOMED_REQUIRE(h->hcache.full(), MOMED_ESTATE, "hit cache: the block map needs a full cache");
+    MOMED_REQUIRE(h->hcache.full(), MOMED_ESTATE, "hit cache: the block map needs the hit records");
     const HitCacheView hv = h->hcache.view();
     const OpView ov = h->op.view();
     const bool hb = (u != nullptr) && (std::is_same<R, double>::value ? ov.t_ampb != nullptr : ov.t_ampb32 != nullptr);

@@ -161,6 +161,8 @@ void build_index(momed_handle* h) {
     MOMED_CUDA_TRY(cudaMemcpyAsync(ranges.data(), dr.p, ranges.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
 
+    h->basis_pop_max = ranges[3];          // at L = 0 the high part is the whole state
+
     // choose the split minimising table entries; widen popcount ranges by the largest
     // change a term can make so that every target of a hit maps into the tables
     int best_L = -1;

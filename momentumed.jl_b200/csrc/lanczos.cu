@@ -52,6 +52,11 @@ void apply_h(momed_handle* h, const double2* x, double2* y) {
         prof_end(h, MOMED_KERNEL_SPMV_C128);
         return;
     }
+    if (h->hcache.pair.built) {
+        launch_pair_c128(h, x, y, h->u, h->stream);
+        prof_end(h, MOMED_KERNEL_HC_MATVEC_C128);
+        return;
+    }
     if (h->hcache.built) {
         launch_matvec_hc_c128(h, x, y, h->op.has_b ? h->u_dev.p : nullptr, h->n, h->stream);
         prof_end(h, MOMED_KERNEL_HC_MATVEC_C128);
@@ -65,6 +70,11 @@ void apply_h(momed_handle* h, const float2* x, float2* y) {
     if (h->sparse.built) {
         launch_spmv_c64(h->sparse, x, y, h->n, h->stream);
         prof_end(h, MOMED_KERNEL_SPMV_C64);
+        return;
+    }
+    if (h->hcache.pair.built) {
+        launch_pair_c64(h, x, y, h->u, h->stream);
+        prof_end(h, MOMED_KERNEL_HC_MATVEC_C64);
         return;
     }
     if (h->hcache.built) {
@@ -405,8 +415,9 @@ using namespace momed;
 int momed_eigsolve_impl(momed_handle* h, const momed_solve_opts* o, const double* vec0, double* vals, double* resid,
                         void* vecs, momed_info* info) {
     if (!h->sparse.built) {                  // a built sparse matrix needs no index or operator check
-        ensure_ready(h);
+        ensure_index(h);
         ensure_hit_cache(h);
+        if (!h->hcache.pair.built) ensure_ready(h);
     }
     const int64_t N = h->n;
     const int nev = (int)std::min<int64_t>(o->nev, N);

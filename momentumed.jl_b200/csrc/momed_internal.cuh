@@ -159,6 +159,7 @@ struct Operator {
     DevBuf<int32_t> g_start, single, pair, generic;
     DevBuf<double2> amp, ampb;
     DevBuf<float2> amp32, ampb32;
+    std::vector<uint64_t> h_in, h_out;   // host copies of t_in and t_out
     OpView view() const;
 };
 
@@ -217,9 +218,69 @@ struct HitCacheView {
     const uint16_t* slot;      // [nnz] slot mode: the term slot of each off-diagonal hit
 };
 
+// Pair classes of the working operator's two-body terms (pairmap.cu).
+struct PairPlanView {
+    int32_t nclass;
+    const int4* cls;           // [nclass] {pairs P, offset in mask/coup, offset in V, 0}
+    const uint64_t* mask;      // pair masks, class by class
+    const uint32_t* coup;      // per pair: the pairs of its class it is coupled to (not itself)
+    const int32_t* ptab;       // [64 * 64] class << 8 | slot of the pair {a < b}, -1: none
+};
+struct PairPlan {
+    int state = -1;            // -1 not looked at, 0 the operator does not take the pair form, 1 ready
+    int nclass = 0, pmax = 0;
+    int64_t nv = 0;            // sum of P * P
+    double density = 0.0;      // share of the off-diagonal couplings that the list has
+    std::vector<int> P;        // pairs of each class
+    DevBuf<int4> cls;
+    DevBuf<uint64_t> mask;
+    DevBuf<uint32_t> coup;
+    DevBuf<int32_t> ptab, vslot, d1;   // vslot [nv] and d1 [64]: term slots of V and the one-body diagonal
+    DevBuf<double2> v64, d64;          // their values at u64 / u32
+    DevBuf<float2> v32, d32;
+    double u64 = 0.0, u32 = 0.0;
+    bool ok64 = false, ok32 = false;
+    PairPlanView view() const;
+};
+// Tables of the pair-factorised map for one basis (pairmap.cu).
+struct PairView {
+    int64_t n;
+    int32_t kmax;              // pairs of a row (the most any row has)
+    const uint4* tile;         // [tiles] {active pairs, first slot, first entry, 0}
+    const uint32_t* ent_row;   // [slots] row | sign << 31, ~0: none
+    const uint32_t* row_ent;   // [kmax][n] entry, ~0: none
+    const int4* work;          // {class, first tile, tiles, 0}
+};
+struct PairMap {
+    bool built = false;
+    bool declined = false;     // looked at for this basis and operator, not worth it
+    int64_t n = 0, entries = 0, hits = 0, bytes = 0;
+    int32_t kmax = 0, nwork = 0;
+    DevBuf<uint4> tile;
+    DevBuf<uint32_t> ent_row, row_ent;
+    DevBuf<int4> work;
+    DevBuf<double2> psi64;     // workspace of a product, one value per entry
+    DevBuf<float2> psi32;
+    PairView view() const;
+    void release() {
+        built = declined = false;
+        n = entries = hits = bytes = 0;
+        kmax = nwork = 0;
+        tile.release();
+        ent_row.release();
+        row_ent.release();
+        work.release();
+        psi64.release();
+        psi32.release();
+    }
+};
+
 struct HitCache {
     bool built = false;
-    int mode = 0;               // 1: full (target and term slot per hit), 2: term slots only
+    int mode = 0;               // 1: full (pair tables, or target and term slot per hit), 2: term slots only
+    bool records = false;       // the hit records are built (the block maps read them)
+    PairMap pair;               // the single-vector map's tables, where the operator takes that form
+    int plain_calls = 0;        // momed_matvec calls on this basis and operator without a cache
     int64_t nnz = 0, bytes = 0;
     double build_ms = 0.0;
     DevBuf<int64_t> row_ptr;
@@ -234,9 +295,20 @@ struct HitCache {
     double comb_u64 = 0.0, comb_u32 = 0.0;
     bool comb_ok64 = false, comb_ok32 = false;
     HitCacheView view() const;
-    bool full() const { return built && mode == 1; }   // the block maps read full caches only
+    void release_records() {
+        records = false;
+        seg.release();
+        hit.release();
+        row_ptr.release();
+        dg64.release();
+        dg32.release();
+    }
+    bool full() const { return built && records; }     // the block maps read hit records only
     void release() {
         built = false;
+        records = false;
+        pair.release();
+        plain_calls = 0;
         mode = 0;
         nnz = bytes = 0;
         slot.release();
@@ -270,10 +342,12 @@ struct momed_handle {
     int64_t n = 0;                         // basis size
     momed::DevBuf<uint64_t> basis;
     uint64_t basis_or = 0;                 // OR of all basis states
+    int32_t basis_pop_max = 0;             // most particles of a basis state (set with the index)
     momed::Index index;
     bool index_dirty = true;
     uint64_t index_bits = 0;               // bits the index tables cover
     momed::Operator op;
+    momed::PairPlan pplan;                 // pair classes of op
     std::vector<int64_t> op_order;         // device term slot q holds entry op_order[q] of the uploaded list
     momed::TwoBodyRecipe recipe;           // amplitudes regenerated on the device (momed_set_kshift)
     int32_t block_solver = -1;             // -1: the block solver when it pays, 0: single-vector only
@@ -315,6 +389,7 @@ const uint32_t* device_binomials();
 
 // index.cu
 void build_index(momed_handle* h);
+void ensure_index(momed_handle* h);            // abi.cu: the index tables of the working basis
 IndexView index_view(const momed_handle* h);
 int64_t validate_operator(momed_handle* h);   // counts (row, term) targets missing from the basis
 
@@ -322,8 +397,12 @@ int64_t validate_operator(momed_handle* h);   // counts (row, term) targets miss
 int64_t hit_cache_bytes(int64_t n, int64_t hits);
 int64_t slot_cache_bytes(int64_t n, int64_t hits);
 int hit_cache_wanted(const momed_handle* h);             // 0 none, 1 full, 2 term slots only
-void build_hit_cache(momed_handle* h, int mode = 1);
+void build_hit_cache(momed_handle* h, int mode = 1);     // mode 1: pair tables where possible, else records
 void ensure_hit_cache(momed_handle* h);
+void build_hit_records(momed_handle* h);                 // the records of a built full cache, if missing
+void ensure_hit_records(momed_handle* h);                // before block maps: under the automatic size rule
+void ensure_plain_pair(momed_handle* h);                 // pair tables for repeated momed_matvec calls
+int64_t full_cache_bytes(momed_handle* h, bool block_maps);   // what a full cache will hold
 void launch_matvec_hc_c128(momed_handle* h, const double2* x, double2* y, const double* u, int64_t rows,
                            cudaStream_t st);
 void launch_matvec_hc_c64(momed_handle* h, const float2* x, float2* y, const float* u, int64_t rows,
@@ -332,6 +411,13 @@ void launch_block_hc_c64(const momed_handle* h, const float2* x, float2* y, cons
                          cudaStream_t st);
 void launch_block_hc_c128(const momed_handle* h, const double2* x, double2* y, const double* u, int32_t nb,
                           int64_t rows, cudaStream_t st);
+
+// pairmap.cu
+bool pair_possible(momed_handle* h);           // operator and basis take the pair form
+int64_t pair_bytes(const momed_handle* h);     // its device memory, FP64 workspace included
+bool build_pair_map(momed_handle* h);          // false: declined
+void launch_pair_c128(momed_handle* h, const double2* x, double2* y, double u, cudaStream_t st);
+void launch_pair_c64(momed_handle* h, const float2* x, float2* y, double u, cudaStream_t st);
 
 // matvec.cu
 void launch_matvec_c128(const IndexView& iv, const OpView& ov, const double2* x, double2* y,

@@ -298,7 +298,7 @@ void worker_loop(momed_server* S, int slot) {
                 std::lock_guard<std::mutex> lk(S->mu);
                 S->op_hits_per_row[r->op] = (double)h->nnz / (double)N;
                 if (knob("MOMED_SERVE_HITCACHE", "1") != "0") {
-                    const int64_t need = hit_cache_bytes(N, h->nnz);
+                    const int64_t need = full_cache_bytes(h, nu > 1);
                     if (S->used + need <= S->budget) {
                         S->used += need;
                         hc_bytes = need;
@@ -335,7 +335,8 @@ void worker_loop(momed_server* S, int slot) {
             try {
                 if (hc_bytes > 0) {
                     try {
-                        build_hit_cache(h, hc_mode);
+                        if (nu > 1 && hc_mode == 1) build_hit_records(h);
+                        else build_hit_cache(h, hc_mode);
                     } catch (const Error& e) {
                         if (e.code != MOMED_ENOMEM) throw;
                         unreserve();          // the device is shorter than the budget: candidate map

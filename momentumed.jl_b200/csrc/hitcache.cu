@@ -772,8 +772,33 @@ template <> struct CombSlot<float> {
     static bool& ok(HitCache& c) { return c.comb_ok32; }
 };
 
-// u is the handle's parameter on the device (h->u_dev / u_dev32): the combined amplitudes are
-// formed again whenever the handle's u differs from the one they were formed at.
+// The term amplitudes at the handle's parameter (A, or A + u B).  u is that parameter on the device
+// (h->u_dev / u_dev32): the combined amplitudes are formed again whenever the handle's u differs
+// from the one they were formed at.
+template <typename R>
+static const typename Cx<R>::T* combined_amp(momed_handle* h, const R* u, bool hb, cudaStream_t st) {
+    const OpView ov = h->op.view();
+    const typename Cx<R>::T* amp = amp_a_host<R>(ov);
+    if (!hb) return amp;
+    HitCache& hc = h->hcache;
+    auto& cb = CombSlot<R>::buf(hc);
+    if (!CombSlot<R>::ok(hc) || CombSlot<R>::u(hc) != h->u) {
+        const int64_t n = ov.nterms;
+        cb.resize(std::max<int64_t>(n, 1));
+        const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 1184));
+        k_hc_combine<R><<<g, 256, 0, st>>>(amp, amp_b_host<R>(ov), u, cb.p, n);
+        MOMED_CUDA_TRY(cudaGetLastError());
+        note_launches(1);
+        CombSlot<R>::u(hc) = h->u;
+        CombSlot<R>::ok(hc) = true;
+    }
+    return cb.p;
+}
+
+const double2* hit_amplitudes_c128(momed_handle* h, cudaStream_t st) {
+    return combined_amp<double>(h, h->u_dev.p, h->op.has_b, st);
+}
+
 template <typename R>
 static void matvec_hc_dispatch(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* y, const R* u,
                                int64_t rows, cudaStream_t st) {
@@ -782,23 +807,8 @@ static void matvec_hc_dispatch(momed_handle* h, const typename Cx<R>::T* x, type
     const HitCacheView hv = h->hcache.view();
     const OpView ov = h->op.view();
     const bool hb = (u != nullptr) && (std::is_same<R, double>::value ? ov.t_ampb != nullptr : ov.t_ampb32 != nullptr);
-    const C2* amp = amp_a_host<R>(ov);
     MOMED_REQUIRE(h->hcache.built, MOMED_ESTATE, "hit cache: not built");
-    if (hb) {
-        HitCache& hc = h->hcache;
-        auto& cb = CombSlot<R>::buf(hc);
-        if (!CombSlot<R>::ok(hc) || CombSlot<R>::u(hc) != h->u) {
-            const int64_t n = ov.nterms;
-            cb.resize(std::max<int64_t>(n, 1));
-            const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 1184));
-            k_hc_combine<R><<<g, 256, 0, st>>>(amp, amp_b_host<R>(ov), u, cb.p, n);
-            MOMED_CUDA_TRY(cudaGetLastError());
-            note_launches(1);
-            CombSlot<R>::u(hc) = h->u;
-            CombSlot<R>::ok(hc) = true;
-        }
-        amp = cb.p;
-    }
+    const C2* amp = combined_amp<R>(h, u, hb, st);
     if (h->hcache.mode == 2) {
         const IndexView iv = index_view(h);
         auto gs = [&](auto k, const R* up) { k<<<hc_grid(k, rows), kWarps * 32, 0, st>>>(iv, hv, ov, amp, x, y, up, rows); };

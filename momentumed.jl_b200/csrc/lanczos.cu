@@ -24,7 +24,7 @@
 #include <complex>
 #include <cstring>
 
-#include "vecops.cuh"
+#include "cycle.cuh"
 
 namespace momed {
 
@@ -108,8 +108,17 @@ struct Lanczos {
     int grid;
     DevBuf<VT> V;
     DevBuf<double2> partial, coefA, coefB;
-    DevBuf<double> scal, alpha, beta, Ud;
+    DevBuf<double> scal, ab, Ud;     // ab: alpha [m], beta [m]
+    double *alpha, *beta;
     DevBuf<int> flag;
+    std::vector<double> Uc;          // restart coefficients, alive until their copy has run
+    // cooperative steps (cycle.cu): FP64 without per-launch timing
+    int coop = -1;                   // CycleMap, -1: the separate kernels
+    int coop_grid = 0;
+    CycleArgs ca{};
+    DevBuf<double2> cpart, xbuf;
+    DevBuf<double> npart;
+    DevBuf<unsigned> bar;
 
     Lanczos(momed_handle* hh, int mm) : h(hh), N(hh->n), m(mm), st(hh->stream) {
         grid = vec_grid(N);
@@ -118,12 +127,80 @@ struct Lanczos {
         coefA.resize(kMaxCols + 1);
         coefB.resize(kMaxCols + 1);
         scal.resize(4);
-        alpha.resize(m);
-        beta.resize(m);
+        ab.resize(2 * m);
+        alpha = ab.p;
+        beta = ab.p + m;
         Ud.resize((size_t)m * m);
         flag.resize(1);
+        if constexpr (std::is_same<VT, double2>::value) plan_coop();
     }
     VT* col(int i) { return V.p + (size_t)i * N; }
+
+    // The map inside the cooperative kernel: CSR and hit records.  Beside the pair map each step's
+    // orthogonalisation runs as one.  Candidate and slot-mode maps keep the separate kernels.
+    void plan_coop() {
+        const char* e = std::getenv("MOMED_COOP");
+        if ((e && e[0] == '0') || h->prof) return;
+        if (h->sparse.built) coop = CYCLE_CSR;
+        else if (h->hcache.pair.built) coop = CYCLE_NONE;
+        else if (h->hcache.full()) coop = CYCLE_HITS;
+        if (coop < 0 || !cycle_plan(N, ca, coop_grid)) {
+            coop = -1;
+            return;
+        }
+        cpart.resize((size_t)coop_grid * (kMaxCols + 1));
+        npart.resize(coop_grid);
+        bar.resize(3);                   // barrier, its exits, the error flag
+        MOMED_CUDA_TRY(cudaMemsetAsync(bar.p, 0, 3 * sizeof(unsigned), st));
+        if (coop != CYCLE_NONE) xbuf.resize((size_t)2 * N);
+        ca.part = cpart.p;
+        ca.npart = npart.p;
+        ca.xbuf = xbuf.p;
+        ca.alpha = alpha;
+        ca.beta = beta;
+        ca.bar = bar.p;
+        ca.err = reinterpret_cast<int*>(bar.p + 2);
+        if (coop == CYCLE_CSR) {
+            ca.row_ptr = h->sparse.row_ptr.p;
+            ca.col = h->sparse.col.p;
+            ca.val = h->sparse.val.p;
+        } else if (coop == CYCLE_HITS) {
+            const HitCacheView hv = h->hcache.view();
+            ca.row_ptr = hv.row_ptr;
+            ca.hit = hv.hit;
+            ca.dg = hv.dg64;
+            ca.has_b = h->op.has_b ? 1 : 0;
+            ca.u = h->u;
+            ca.amp = hit_amplitudes_c128(h, st);
+        }
+    }
+    void coop_steps(int j0, int j1) {
+        if constexpr (std::is_same<VT, double2>::value) {
+            ca.V = V.p;
+            ca.j0 = j0;
+            ca.j1 = j1;
+            launch_cycle(ca, coop, coop_grid, st);
+        }
+    }
+    // steps [j0, j1)
+    void steps(int j0, int j1) {
+        if (coop > CYCLE_NONE && j1 > j0) {
+            coop_steps(j0, j1);
+            return;
+        }
+        for (int j = j0; j < j1; ++j) step(j);
+    }
+    // alpha and beta on the host; a barrier that gave up ends the solve
+    void fetch(double* ha, double* hb) {
+        int err = 0;
+        std::vector<double> t((size_t)2 * m);
+        MOMED_CUDA_TRY(cudaMemcpyAsync(t.data(), ab.p, t.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (coop >= 0) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, ca.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+        if (err) throw Error{MOMED_ETIMEOUT, "Lanczos cycle: a grid barrier gave up"};
+        std::copy(t.begin(), t.begin() + m, ha);
+        std::copy(t.begin() + m, t.end(), hb);
+    }
 
     void normalize(VT* v) {
         vec_proj<VT>(v, N, 0, v, partial.p, grid, nullptr, st);
@@ -144,6 +221,10 @@ struct Lanczos {
     void step(int j) {
         VT* w = col(j + 1);
         apply_h(h, col(j), w);
+        if (coop == CYCLE_NONE) {
+            coop_steps(j, j + 1);
+            return;
+        }
         const int nc = j + 1;
         vec_proj<VT>(V.p, N, nc, w, partial.p, grid, nullptr, st);
         vec_reduce(partial.p, grid, nc + 1, coefA.p, nullptr, st);
@@ -152,7 +233,7 @@ struct Lanczos {
         vec_proj<VT>(V.p, N, nc, w, partial.p, grid, flag.p, st);
         vec_reduce(partial.p, grid, nc + 1, coefB.p, flag.p, st);
         vec_update<VT>(V.p, N, nc, coefB.p, w, partial.p, grid, flag.p, st);
-        vec_finalize(coefA.p, coefB.p, nc, partial.p, grid, flag.p, scal.p, alpha.p, beta.p, j, st);
+        vec_finalize(coefA.p, coefB.p, nc, partial.p, grid, flag.p, scal.p, alpha, beta, j, st);
         vec_scale<VT>(w, N, scal.p, st);
     }
 
@@ -173,10 +254,9 @@ struct Lanczos {
         for (;;) {
             int jstart = k;
             int mm = m;
-            for (int j = jstart; j < m; ++j) { step(j); ++matvecs; }
-            MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, m * sizeof(double), cudaMemcpyDeviceToHost, st));
-            MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, m * sizeof(double), cudaMemcpyDeviceToHost, st));
-            MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+            steps(jstart, m);
+            matvecs += m - jstart;
+            fetch(ha.data(), hb.data());
             // invariant-subspace breakdown inside the cycle
             double scale = 0.0;
             for (int j = k; j < m; ++j) scale = std::max(scale, std::fabs(ha[j]));
@@ -189,11 +269,10 @@ struct Lanczos {
                     orthonormalize(col(j + 1), j + 1);
                     hb[j] = 0.0;
                     double zero = 0.0;
-                    MOMED_CUDA_TRY(cudaMemcpyAsync(beta.p + j, &zero, sizeof(double), cudaMemcpyHostToDevice, st));
-                    for (int jj = j + 1; jj < m; ++jj) { step(jj); ++matvecs; }
-                    MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, m * sizeof(double), cudaMemcpyDeviceToHost, st));
-                    MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, m * sizeof(double), cudaMemcpyDeviceToHost, st));
-                    MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+                    MOMED_CUDA_TRY(cudaMemcpyAsync(beta + j, &zero, sizeof(double), cudaMemcpyHostToDevice, st));
+                    steps(j + 1, m);
+                    matvecs += m - j - 1;
+                    fetch(ha.data(), hb.data());
                     hb[j] = 0.0;
                 }
             }
@@ -227,7 +306,7 @@ struct Lanczos {
                 int nv = std::min(nwant, mm);
                 out.kept = nv;
                 if (vectors && nv > 0) {
-                    std::vector<double> Uc((size_t)mm * nv);
+                    Uc.assign((size_t)mm * nv, 0.0);
                     for (int i = 0; i < nv; ++i)
                         for (int a = 0; a < mm; ++a) Uc[(size_t)i * mm + a] = U[(size_t)a * mm + i];
                     MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, Uc.data(), Uc.size() * 8, cudaMemcpyHostToDevice, st));
@@ -241,7 +320,7 @@ struct Lanczos {
             keep = std::max(keep, nev);
             keep = std::min(keep, m - 2);
             keep = std::max(keep, 1);
-            std::vector<double> Uc((size_t)m * keep);
+            Uc.assign((size_t)m * keep, 0.0);
             for (int i = 0; i < keep; ++i)
                 for (int a = 0; a < m; ++a) Uc[(size_t)i * m + a] = U[(size_t)a * m + i];
             MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, Uc.data(), Uc.size() * 8, cudaMemcpyHostToDevice, st));
@@ -250,8 +329,7 @@ struct Lanczos {
             arrow.resize(keep);
             for (int i = 0; i < keep; ++i) arrow[i] = beta_last * U[(size_t)(m - 1) * m + i];
             k = keep;
-            ++restarts;
-            MOMED_CUDA_TRY(cudaStreamSynchronize(st));   // Uc must outlive the async copy
+            ++restarts;                      // Uc is written again after the next fetch
         }
     }
 };

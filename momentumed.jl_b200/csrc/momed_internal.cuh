@@ -403,6 +403,7 @@ void build_hit_records(momed_handle* h);                 // the records of a bui
 void ensure_hit_records(momed_handle* h);                // before block maps: under the automatic size rule
 void ensure_plain_pair(momed_handle* h);                 // pair tables for repeated momed_matvec calls
 int64_t full_cache_bytes(momed_handle* h, bool block_maps);   // what a full cache will hold
+const double2* hit_amplitudes_c128(momed_handle* h, cudaStream_t st);   // at the handle's u
 void launch_matvec_hc_c128(momed_handle* h, const double2* x, double2* y, const double* u, int64_t rows,
                            cudaStream_t st);
 void launch_matvec_hc_c64(momed_handle* h, const float2* x, float2* y, const float* u, int64_t rows,

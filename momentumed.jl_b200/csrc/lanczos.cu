@@ -130,7 +130,7 @@ struct Lanczos {
         ab.resize(2 * m);
         alpha = ab.p;
         beta = ab.p + m;
-        Ud.resize((size_t)m * m);
+        Ud.resize((size_t)m * (m + 8));      // packed in groups of up to 8 outputs
         flag.resize(1);
         if constexpr (std::is_same<VT, double2>::value) plan_coop();
     }
@@ -309,6 +309,8 @@ struct Lanczos {
                     Uc.assign((size_t)mm * nv, 0.0);
                     for (int i = 0; i < nv; ++i)
                         for (int a = 0; a < mm; ++a) Uc[(size_t)i * mm + a] = U[(size_t)a * mm + i];
+                    Uc = vec_pack_coefs(Uc, mm, nv);
+                    Ud.resize(Uc.size());
                     MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, Uc.data(), Uc.size() * 8, cudaMemcpyHostToDevice, st));
                     vec_combine<VT, double2>(V.p, N, mm, Ud.p, nv, vectors, N, -1, st);
                     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
@@ -323,6 +325,7 @@ struct Lanczos {
             Uc.assign((size_t)m * keep, 0.0);
             for (int i = 0; i < keep; ++i)
                 for (int a = 0; a < m; ++a) Uc[(size_t)i * m + a] = U[(size_t)a * m + i];
+            Uc = vec_pack_coefs(Uc, m, keep);
             MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, Uc.data(), Uc.size() * 8, cudaMemcpyHostToDevice, st));
             vec_combine<VT, VT>(V.p, N, m, Ud.p, keep, V.p, N, m, st);
             kept_theta.assign(th.begin(), th.begin() + keep);
@@ -587,10 +590,10 @@ int momed_eigsolve_impl(momed_handle* h, const momed_solve_opts* o, const double
             // phase 3: FP64 Lanczos warm-started from the refined vectors
             DevBuf<double2> sv;
             sv.resize(N);
-            std::vector<double> ones(kk, 1.0);
+            const std::vector<double> ones = vec_pack_coefs(std::vector<double>(kk, 1.0), kk, 1);
             DevBuf<double> Ud;
-            Ud.resize(kk);
-            MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, ones.data(), kk * 8, cudaMemcpyHostToDevice, st));
+            Ud.resize(ones.size());
+            MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, ones.data(), ones.size() * 8, cudaMemcpyHostToDevice, st));
             vec_combine<double2, double2>(X1.p, N, kk, Ud.p, 1, sv.p, N, -1, st);
             MOMED_CUDA_TRY(cudaStreamSynchronize(st));
             Lanczos<double2> L(h, m);

@@ -193,39 +193,70 @@ __global__ void k_random(VT* v, int64_t N, uint64_t seed) {
         v[n] = from_d2<VT>(make_double2(u01(seed, 2 * (uint64_t)n), u01(seed, 2 * (uint64_t)n + 1)));
 }
 
-// Tile of TR rows of all m (+1) columns staged in shared memory, then every
-// (row, output) pair is a length-m dot product from shared memory.
-template <typename VIN, typename VOUT, int TR>
+// out[:, i] = sum_a U[a][i] V[:, a].  A tile of TR rows of all m (+1) columns is staged in shared
+// memory (so out may overlap V); a warp then forms OC outputs of TR / 32 rows per lane in registers.
+// Bound by shared memory: per column a warp reads its lanes' values (4 wavefronts a row) and OC
+// coefficients (broadcast) for 2 OC TR / 32 FMAs; one output per thread, as before, read 16 bytes for
+// every 2 FMAs and ran at 12% of the copy peak.  Restart of a 1.0M-state basis, 64 columns to 39: 2.18
+// -> 1.02 ms; 174k states, 30 to 18: 115 -> 47 us.
+// U packed by groups of OC outputs: U[(g * m + a) * OC + k], zero beyond nout.
+template <typename VIN, typename VOUT, int OC>
 __global__ void __launch_bounds__(kVecThreads)
 k_combine(const VIN* V, int64_t N, int m, const double* __restrict__ U, int nout, VOUT* out, int64_t out_ld,
           int copy_col) {
+    constexpr int TR = 64, RL = TR / 32;
     extern __shared__ double2 tile[];   // [(m + 1) * TR]
     const int ncopy = copy_col >= 0 ? 1 : 0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int groups = (nout + OC - 1) / OC;
     for (int64_t t0 = (int64_t)blockIdx.x * TR; t0 < N; t0 += (int64_t)gridDim.x * TR) {
         const int rows = (int)((N - t0) < (int64_t)TR ? (N - t0) : (int64_t)TR);
 #pragma unroll 4
-        for (int e = threadIdx.x; e < (m + ncopy) * TR; e += blockDim.x) {
-            int a = e / TR, r = e % TR;
-            int col = (a < m) ? a : copy_col;
+        for (int e = threadIdx.x; e < (m + ncopy) * TR; e += kVecThreads) {
+            const int a = e / TR, r = e % TR;
+            const int col = (a < m) ? a : copy_col;
             tile[e] = (r < rows) ? to_d2(V[(int64_t)col * N + t0 + r]) : make_double2(0.0, 0.0);
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < nout * TR; e += blockDim.x) {
-            int i = e / TR, r = e % TR;
-            if (r < rows) {
-                double sx = 0.0, sy = 0.0;
-                const double* u = U + (int64_t)i * m;
-                for (int a = 0; a < m; ++a) {
-                    double2 v = tile[a * TR + r];
-                    double c = __ldg(u + a);
-                    sx += c * v.x;
-                    sy += c * v.y;
+        for (int g = wid; g < groups; g += kVecThreads / 32) {
+            double ax[RL][OC], ay[RL][OC];
+#pragma unroll
+            for (int j = 0; j < RL; ++j)
+#pragma unroll
+                for (int k = 0; k < OC; ++k) { ax[j][k] = 0.0; ay[j][k] = 0.0; }
+            const double* u = U + (int64_t)g * m * OC;
+            const double2* v = tile + lane;
+#pragma unroll 2
+            for (int a = 0; a < m; ++a, u += OC, v += TR) {
+                double c[OC];
+#pragma unroll
+                for (int k = 0; k < OC; k += 2) {
+                    const double2 cc = __ldg(reinterpret_cast<const double2*>(u + k));
+                    c[k] = cc.x;
+                    c[k + 1] = cc.y;
                 }
-                out[(int64_t)i * out_ld + t0 + r] = from_d2<VOUT>(make_double2(sx, sy));
+#pragma unroll
+                for (int j = 0; j < RL; ++j) {
+                    const double2 x = v[32 * j];
+#pragma unroll
+                    for (int k = 0; k < OC; ++k) {
+                        ax[j][k] += c[k] * x.x;
+                        ay[j][k] += c[k] * x.y;
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < OC; ++k) {
+                const int i = g * OC + k;
+                if (i >= nout) break;
+#pragma unroll
+                for (int j = 0; j < RL; ++j)
+                    if (lane + 32 * j < rows)
+                        out[(int64_t)i * out_ld + t0 + lane + 32 * j] = from_d2<VOUT>(make_double2(ax[j][k], ay[j][k]));
             }
         }
         if (ncopy) {
-            for (int r = threadIdx.x; r < rows; r += blockDim.x)
+            for (int r = threadIdx.x; r < rows; r += kVecThreads)
                 out[(int64_t)nout * out_ld + t0 + r] = from_d2<VOUT>(tile[m * TR + r]);
         }
         __syncthreads();
@@ -349,6 +380,16 @@ void vec_random(VT* v, int64_t N, uint64_t seed, cudaStream_t st) {
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
 }
+int vec_combine_group(int nout) { return nout >= 24 ? 8 : 4; }
+
+std::vector<double> vec_pack_coefs(const std::vector<double>& U, int m, int nout) {
+    const int oc = vec_combine_group(nout);
+    std::vector<double> P((size_t)((nout + oc - 1) / oc) * m * oc, 0.0);
+    for (int i = 0; i < nout; ++i)
+        for (int a = 0; a < m; ++a) P[((size_t)(i / oc) * m + a) * oc + i % oc] = U[(size_t)i * m + a];
+    return P;
+}
+
 template <typename VIN, typename VOUT>
 void vec_combine(const VIN* V, int64_t N, int m, const double* U, int nout, VOUT* out, int64_t out_ld, int copy_col,
                  cudaStream_t st) {
@@ -356,23 +397,18 @@ void vec_combine(const VIN* V, int64_t N, int m, const double* U, int nout, VOUT
     // largest tile the kernel can get, so callers on other threads never lower it under a launch.
     const int ncopy = copy_col >= 0 ? 1 : 0;
     MOMED_REQUIRE(m + ncopy <= kMaxCols + 1, MOMED_EINVAL, "krylovdim too large");
-    if (m + ncopy <= 100) {
-        constexpr int TR = 64;
-        size_t smem = (size_t)(m + ncopy) * TR * sizeof(double2);
-        auto k = k_combine<VIN, VOUT, TR>;
-        MOMED_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)(100 * TR * sizeof(double2))));
-        int grid = (int)std::max<int64_t>(1, std::min<int64_t>((N + TR - 1) / TR, (int64_t)sm_count() * 2));
-        k<<<grid, kVecThreads, smem, st>>>(V, N, m, U, nout, out, out_ld, copy_col);
-    } else {
-        constexpr int TR = 32;
-        size_t smem = (size_t)(m + ncopy) * TR * sizeof(double2);
-        auto k = k_combine<VIN, VOUT, TR>;
+    constexpr int TR = 64;
+    const size_t smem = (size_t)(m + ncopy) * TR * sizeof(double2);
+    auto go = [&](auto k) {
         MOMED_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)((kMaxCols + 1) * TR * sizeof(double2))));
-        int grid = (int)std::max<int64_t>(1, std::min<int64_t>((N + TR - 1) / TR, (int64_t)sm_count() * 2));
+        // resident blocks: registers allow three, shared memory fewer for wide bases
+        const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(3, (size_t)220 * 1024 / (smem + 1024)));
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((N + TR - 1) / TR, (int64_t)sm_count() * per_sm));
         k<<<grid, kVecThreads, smem, st>>>(V, N, m, U, nout, out, out_ld, copy_col);
-    }
+    };
+    if (vec_combine_group(nout) == 8) go(k_combine<VIN, VOUT, 8>);
+    else go(k_combine<VIN, VOUT, 4>);
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
 }

@@ -52,8 +52,10 @@ template <typename VT>
 void vec_scale(VT* v, int64_t N, const double* scal, cudaStream_t st);
 template <typename VT>
 void vec_random(VT* v, int64_t N, uint64_t seed, cudaStream_t st);
-// out[:, i] = sum_a U[a + i*m] V[:, a] for i < nout (U column-major m x nout, FP64);
-// when copy_col >= 0 also out[:, nout] = V[:, copy_col].  In place (out == V) is allowed.
+// out[:, i] = sum_a U[a + i*m] V[:, a] for i < nout (U column-major m x nout, FP64, on the device as
+// vec_pack_coefs lays it out); when copy_col >= 0 also out[:, nout] = V[:, copy_col].  In place
+// (out == V) is allowed.
+std::vector<double> vec_pack_coefs(const std::vector<double>& U, int m, int nout);
 template <typename VIN, typename VOUT>
 void vec_combine(const VIN* V, int64_t N, int m, const double* U, int nout, VOUT* out, int64_t out_ld, int copy_col,
                  cudaStream_t st);

@@ -270,22 +270,8 @@ void keep_pool_memory(int device) {
     done.push_back(device);
 }
 
-__global__ void k_or_basis(const uint64_t* b, int64_t n, unsigned long long* out) {
-    uint64_t acc = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        acc |= b[i];
-    for (int o = 16; o > 0; o >>= 1) acc |= __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && acc) atomicOr(out, (unsigned long long)acc);
-}
-
 void after_basis_change(momed_handle* h) {
-    h->counters.resize(16);
-    MOMED_CUDA_TRY(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(unsigned long long), h->stream));
-    if (h->n > 0) k_or_basis<<<std::min<int64_t>(1184, (h->n + 255) / 256), 256, 0, h->stream>>>(h->basis.p, h->n, h->counters.p + 2);
-    unsigned long long v = 0;
-    MOMED_CUDA_TRY(cudaMemcpyAsync(&v, h->counters.p + 2, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
-    MOMED_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    h->basis_or = v;
+    scan_basis(h);
     h->index_dirty = true;
     h->op_validated = false;
     h->sparse.release();
@@ -654,6 +640,7 @@ int momed_set_sparse_csr(momed_handle* h, int64_t n, const int64_t* row_ptr, con
         h->basis.release();
         h->n = n;
         h->basis_or = 0;
+        h->basis_scanned = false;
         h->index_dirty = true;
         h->op_validated = false;
         h->sparse_only = true;

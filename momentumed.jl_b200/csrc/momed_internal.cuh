@@ -342,7 +342,11 @@ struct momed_handle {
     int64_t n = 0;                         // basis size
     momed::DevBuf<uint64_t> basis;
     uint64_t basis_or = 0;                 // OR of all basis states
-    int32_t basis_pop_max = 0;             // most particles of a basis state (set with the index)
+    int32_t basis_pop_max = 0;             // most particles of a basis state
+    int64_t basis_bad = 0;                 // places where the basis does not ascend
+    int basis_range[65 * 4] = {};          // per split point: popcount ranges of the low and the high part
+    bool basis_scanned = false;            // the facts above are those of the working basis
+    momed::DevBuf<unsigned char> scan;
     momed::Index index;
     bool index_dirty = true;
     uint64_t index_bits = 0;               // bits the index tables cover
@@ -389,6 +393,7 @@ const uint32_t* device_binomials();
 
 // index.cu
 void build_index(momed_handle* h);
+void scan_basis(momed_handle* h);
 void ensure_index(momed_handle* h);            // abi.cu: the index tables of the working basis
 IndexView index_view(const momed_handle* h);
 int64_t validate_operator(momed_handle* h);   // counts (row, term) targets missing from the basis

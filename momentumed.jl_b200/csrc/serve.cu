@@ -267,6 +267,7 @@ void worker_loop(momed_server* S, int slot) {
             h->op_validated = false;
             h->basis_or = 0;
             for (uint64_t v : r->basis) h->basis_or |= v;
+            h->basis_scanned = false;
             if (cur_op != r->op) {
                 cur_op = -1;
                 upload_operator(h, op.amp_a.data(), op.has_b ? op.amp_b.data() : nullptr, op.in.data(),

@@ -7,9 +7,14 @@
 // sign (-1)^(scat_occ_number(mid, i) + scat_occ_number(mid, j)) where scat_occ_number counts
 // the occupied orbitals above the given one; then rdm[i][j] = conj(rdm[j][i]) for i > j.
 //
-// One thread per basis state walks its occupied orbitals j and the orbitals i <= j; targets are
-// looked up with key checks (c+_i c_j usually leaves a momentum sector).  A block accumulates its
-// norb x norb matrix in shared memory; the host adds the blocks' matrices in block order.
+// One thread per basis state walks its occupied orbitals j and the empty orbitals i < j; targets are
+// looked up with key checks (c+_i c_j usually leaves a momentum sector), and those in the basis add to
+// the block's norb x norb matrix in shared memory.  The occupations (i = j), which every state has,
+// are summed across the warp orbital by orbital instead: as shared-memory atomics, all lanes on the
+// same few diagonal elements, they took most of the kernel (345 us on a 174k-state sector of 27
+// orbitals, 163 without them).  What is left waits for the lookups' table reads, so three blocks of 16
+// warps share an SM (126 us; two of 8 before).  A second kernel adds the blocks' matrices (the host
+// did, after copying all of them: 3.4 MB).
 #include "candidates.cuh"
 
 namespace momed {
@@ -17,8 +22,9 @@ namespace momed {
 namespace {
 
 constexpr int kRdmThreads = 256;
+constexpr int kRdm1Threads = 512;
 
-__global__ void __launch_bounds__(kRdmThreads)
+__global__ void __launch_bounds__(kRdm1Threads)
 k_rdm1(IndexView iv, const double2* __restrict__ psi, int norb, double2* __restrict__ partial) {
     extern __shared__ double2 acc[];                  // [norb * norb]
     __shared__ SharedTables sh;
@@ -26,23 +32,37 @@ k_rdm1(IndexView iv, const double2* __restrict__ psi, int norb, double2* __restr
     for (int e = threadIdx.x; e < nn; e += blockDim.x) acc[e] = make_double2(0.0, 0.0);
     stage_tables(sh, iv);                             // ends with __syncthreads
     const uint64_t omask = norb >= 64 ? ~0ull : ((1ull << norb) - 1ull);
-    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < iv.n; x += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t s = __ldg(iv.basis + x);
-        const double2 pin = __ldg(psi + x);
+    const int lane = threadIdx.x & 31;
+    double occ0 = 0.0, occ1 = 0.0;                    // occupations of orbitals lane and lane + 32
+    for (int64_t x0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); x0 < iv.n;
+         x0 += (int64_t)gridDim.x * blockDim.x) {     // warp-uniform
+        const int64_t x = x0 + lane;
+        const bool in = x < iv.n;
+        const uint64_t s = in ? __ldg(iv.basis + x) : 0ull;
+        const double2 pin = in ? __ldg(psi + x) : make_double2(0.0, 0.0);
+        const double p2 = pin.x * pin.x + pin.y * pin.y;
+        for (int o = 0; o < norb; ++o) {
+            const bool has = (s >> o) & 1ull;
+            if (!__any_sync(kFull, has)) continue;
+            double v = has ? p2 : 0.0;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFull, v, d);
+            if (lane == (o & 31)) {
+                if (o < 32) occ0 += v;
+                else occ1 += v;
+            }
+        }
         uint64_t rem = s & omask;
         while (rem) {
             const int j = __ffsll((long long)rem) - 1;
             rem &= rem - 1ull;
             const uint64_t mid = s & ~(1ull << j);
             const uint64_t above_j = j >= 63 ? 0ull : (~0ull << (j + 1));
-            for (int i = 0; i <= j; ++i) {
-                if (i != j && ((mid >> i) & 1ull)) continue;
-                int64_t y = x;
-                if (i != j) {
-                    y = lookup_index(iv, mid | (1ull << i), sh.base_hi, sh.base_lo, sh.binom);
-                    if (y < 0) continue;
-                }
-                const uint64_t above_i = i >= 63 ? 0ull : (~0ull << (i + 1));
+            for (uint64_t free = ~mid & ((1ull << j) - 1ull); free; free &= free - 1ull) {
+                const int i = __ffsll((long long)free) - 1;
+                const int64_t y = lookup_index(iv, mid | (1ull << i), sh.base_hi, sh.base_lo, sh.binom);
+                if (y < 0) continue;
+                const uint64_t above_i = ~0ull << (i + 1);              // i < j <= 63
                 const bool neg = ((__popcll(mid & above_i) + __popcll(mid & above_j)) & 1) != 0;
                 const double2 pout = __ldg(psi + y);
                 double vr = pout.x * pin.x + pout.y * pin.y;      // conj(psi[y]) * psi[x]
@@ -53,8 +73,29 @@ k_rdm1(IndexView iv, const double2* __restrict__ psi, int norb, double2* __restr
             }
         }
     }
+    if (lane < norb) atomicAdd(&acc[lane * norb + lane].x, occ0);
+    if (lane + 32 < norb) atomicAdd(&acc[(lane + 32) * norb + lane + 32].x, occ1);
     __syncthreads();
     for (int e = threadIdx.x; e < nn; e += blockDim.x) partial[(int64_t)blockIdx.x * nn + e] = acc[e];
+}
+
+// out[e] = sum over the blocks of partial[b][e]: a warp per element, its lanes over the blocks in a
+// fixed stride and tree
+__global__ void k_sum_blocks(const double2* __restrict__ partial, int blocks, int count, double2* __restrict__ out) {
+    const int e = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (e >= count) return;
+    double2 s = make_double2(0.0, 0.0);
+    for (int b = lane; b < blocks; b += 32) {
+        const double2 v = __ldg(partial + (int64_t)b * count + e);
+        s.x += v.x;
+        s.y += v.y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(kFull, s.x, o);
+        s.y += __shfl_xor_sync(kFull, s.y, o);
+    }
+    if (lane == 0) out[e] = s;
 }
 
 // ED_step_inner_prod (MomentumED/src/analysis/manybody_quantum_geometry.jl:48-94): thread per
@@ -124,18 +165,13 @@ void step_inner_prod(momed_handle* h, const double* psi_f, const double* psi_i, 
                                                                           part.p);
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
-    std::vector<double2> hp((size_t)grid * gg);
-    MOMED_CUDA_TRY(cudaMemcpyAsync(hp.data(), part.p, hp.size() * 16, cudaMemcpyDeviceToHost, st));
+    DevBuf<double2> sum;
+    sum.resize(gg);
+    k_sum_blocks<<<(gg + 7) / 8, 256, 0, st>>>(part.p, grid, gg, sum.p);
+    MOMED_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    MOMED_CUDA_TRY(cudaMemcpyAsync(out, sum.p, (size_t)gg * 16, cudaMemcpyDeviceToHost, st));
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-    for (int e = 0; e < gg; ++e) {
-        double re = 0.0, im = 0.0;
-        for (int b = 0; b < grid; ++b) {
-            re += hp[(size_t)b * gg + e].x;
-            im += hp[(size_t)b * gg + e].y;
-        }
-        out[2 * e] = re;
-        out[2 * e + 1] = im;
-    }
 }
 
 void rdm1(momed_handle* h, const double* psi, int norb, double* rdm) {
@@ -163,26 +199,18 @@ void rdm1(momed_handle* h, const double* psi, int norb, double* rdm) {
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kRdmThreads - 1) / kRdmThreads, (int64_t)sms * 2));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + kRdm1Threads - 1) / kRdm1Threads, (int64_t)sms * 3));
     part.resize((size_t)grid * nn);
-    k_rdm1<<<grid, kRdmThreads, smem, st>>>(iv, pd.p, norb, part.p);
+    k_rdm1<<<grid, kRdm1Threads, smem, st>>>(iv, pd.p, norb, part.p);
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
-    std::vector<double2> hp((size_t)grid * nn);
-    MOMED_CUDA_TRY(cudaMemcpyAsync(hp.data(), part.p, hp.size() * 16, cudaMemcpyDeviceToHost, st));
+    DevBuf<double2> sum;
+    sum.resize(nn);
+    k_sum_blocks<<<(nn + 7) / 8, 256, 0, st>>>(part.p, grid, nn, sum.p);
+    MOMED_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    MOMED_CUDA_TRY(cudaMemcpyAsync(rdm, sum.p, (size_t)nn * 16, cudaMemcpyDeviceToHost, st));
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-    for (int i = 0; i < norb; ++i)
-        for (int j = 0; j < norb; ++j) {
-            double re = 0.0, im = 0.0;
-            if (i <= j) {
-                for (int b = 0; b < grid; ++b) {
-                    re += hp[(size_t)b * nn + i * norb + j].x;
-                    im += hp[(size_t)b * nn + i * norb + j].y;
-                }
-            }
-            rdm[2 * ((size_t)i * norb + j)] = re;
-            rdm[2 * ((size_t)i * norb + j) + 1] = im;
-        }
     for (int i = 0; i < norb; ++i)
         for (int j = 0; j < i; ++j) {
             rdm[2 * ((size_t)i * norb + j)] = rdm[2 * ((size_t)j * norb + i)];

@@ -23,7 +23,7 @@
 #include <thread>
 #include <type_traits>
 
-#include "vecops.cuh"
+#include "cycle.cuh"
 
 namespace momed {
 
@@ -455,6 +455,10 @@ struct BlockLanczos {
     std::vector<CycleGraph> graphs;
     bool use_graphs = false;
     int64_t graph_replays = 0;
+    // One right-hand side over the pair map: a step is the map and one cooperative launch (cycle.cu)
+    // instead of the map and eight kernels, and needs no graph.
+    bool coop = false;
+    CycleBufs<VT> cy;
 
     ~BlockLanczos() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
@@ -504,6 +508,8 @@ struct BlockLanczos {
             const char* e = std::getenv("MOMED_GRAPHS");
             use_graphs = !(e && e[0] == '0') && !hh->prof;   // per-launch timing needs eager launches
         }
+        const char* ce = std::getenv("MOMED_COOP");
+        const bool want_coop = NB == 1 && !(ce && ce[0] == '0') && !hh->prof && !hh->sparse.built && hh->hcache.pair.built;
         {   // kernel attributes are set before any capture
             constexpr size_t smem_max = (size_t)kMaxCols * NB * sizeof(double2);
             if (smem_max > 48 * 1024)
@@ -524,6 +530,10 @@ struct BlockLanczos {
         Ud.resize((size_t)NB * m * m);
         flag.resize(NB);
         any.resize(1);
+        if (want_coop && cy.prepare(N, false, alpha.p, beta.p, dgks, st)) {
+            coop = true;
+            use_graphs = false;
+        }
         ud.resize(NB);
         std::vector<RT> uh(NB, (RT)0);
         for (size_t r = 0; r < u.size() && r < (size_t)NB; ++r) uh[r] = (RT)u[r];
@@ -586,6 +596,11 @@ struct BlockLanczos {
     void step(int j) {
         VT* w = col(j + 1);
         BlockMv<VT>::run(h, col(j), w, ud.p, NB, u0);   // counted by its launcher
+        if (coop) {
+            cy.a.keep = dgks;
+            cy.steps(V.p, j, j + 1, CYCLE_NONE, st);
+            return;
+        }
         const int nc = j + 1;
         proj(nc, w, coefA.p, nullptr);
         update(nc, coefA.p, w, nullptr, nullptr);
@@ -668,7 +683,10 @@ struct BlockLanczos {
             }
             MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
             MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
+            int err = 0;
+            if (coop) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
             MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+            CycleBufs<VT>::check(err);
             // per right-hand side projected eigenproblems, in parallel on the host
             auto solve_r = [&](int r) {
                 std::vector<double> T((size_t)m * m, 0.0);
@@ -1329,10 +1347,13 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                     gram(Xb.p, false, k1, g0, nr, gx.p + (size_t)g0 * k1 * NB);          // x_a^H rhs
                     gram(LR.col(k1), true, p, g0, nr, gq.p + (size_t)g0 * p * NB);       // q_j^H rhs
                 }
+                int err = 0;
+                if (LR.coop) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, LR.cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
                 std::vector<double2> hx((size_t)gx_n), hq((size_t)gq_n);
                 MOMED_CUDA_TRY(cudaMemcpyAsync(hx.data(), gx.p, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
                 MOMED_CUDA_TRY(cudaMemcpyAsync(hq.data(), gq.p, hq.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
                 MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+                CycleBufs<float2>::check(err);
                 for (int jr = 0; jr < nrhs; ++jr) {
                     const int i = jr < k1 ? jr : jr - k1;
                     auto& M = jr < k1 ? G : S;

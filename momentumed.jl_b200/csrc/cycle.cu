@@ -1,6 +1,6 @@
-// Lanczos steps of the FP64 single-vector solver as one cooperative kernel.
+// Lanczos steps of the single-vector solvers as one cooperative kernel.
 //
-// A step of lanczos.cu is a map and nine vector kernels (projection, reduction, update, the test
+// A step of lanczos.cu (and of batch.cu with one right-hand side) is a map and nine vector kernels (projection, reduction, update, the test
 // for a second Gram-Schmidt pass, that pass, the norm, the scaling), most of them a few
 // microseconds: on sectors of a few hundred to some ten thousand states a solve spends its time on
 // launches.  Here a block owns a contiguous range of rows for the whole launch and keeps its part of
@@ -22,9 +22,10 @@
 // sectors, the two reads of V on large ones.  One FP64 solve of 4 pairs on the B200, separate kernels
 // / this: 200 states 2.97 / 1.18 ms, 5.5k 8.05 / 3.58, 30.6k 13.1 / 7.1, 104k (hit records) 26.1 /
 // 19.2, 276k (beside the pair map) 41.8 / 34.3, 1.0M 266 / 250: it wins at every size, so the
-// separate kernels stay for what it does not do (FP32, per-launch timing, candidate and slot-mode
-// maps, more rows than the blocks' shared memory holds: 1.89M states).
+// separate kernels stay for what it does not do (per-launch timing, candidate and slot-mode maps,
+// FP32 steps of lanczos.cu, more rows than the blocks' shared memory holds: 1.7M states in FP64).
 #include <algorithm>
+#include <type_traits>
 
 #include "cycle.cuh"
 
@@ -98,7 +99,7 @@ __device__ __forceinline__ double2 ld_rec(const double2* p) {
 
 // w[r] = s * (H x)[r0 + r], a warp per row as k_matvec_hc and k_spmv do it
 template <int MAP>
-__device__ __forceinline__ void cycle_map(const CycleArgs& a, const double2* x, double s, int64_t r0, int nr, double2* w) {
+__device__ __forceinline__ void cycle_map(const CycleArgs<double2>& a, const double2* x, double s, int64_t r0, int nr, double2* w) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int r = wid; r < nr; r += kCW) {
         const int64_t row = r0 + r;
@@ -160,7 +161,8 @@ __device__ __forceinline__ void cycle_map(const CycleArgs& a, const double2* x, 
 }
 
 // part[c][block] = the block's share of V_c^H w for c < ncols (and |w|^2 as c = ncols when norm)
-__device__ __forceinline__ void cycle_proj(const CycleArgs& a, int ncols, bool norm, int64_t r0, int nr, const double2* w,
+template <typename VT>
+__device__ __forceinline__ void cycle_proj(const CycleArgs<VT>& a, int ncols, bool norm, int64_t r0, int nr, const VT* w,
                                            double2* slot) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int ch = a.chunks, len = (nr + ch - 1) / ch, total = (ncols + (norm ? 1 : 0)) * ch;
@@ -169,15 +171,18 @@ __device__ __forceinline__ void cycle_proj(const CycleArgs& a, int ncols, bool n
         const int b = q * len, e = min(nr, b + len);
         double ax = 0.0, ay = 0.0;
         if (c < ncols) {
-            const double2* v = a.V + (int64_t)c * a.N + r0;
+            const VT* v = a.V + (int64_t)c * a.N + r0;
 #pragma unroll 4
             for (int r = b + lane; r < e; r += 32) {
-                const double2 vv = v[r], ww = w[r];
+                const double2 vv = to_d2(v[r]), ww = to_d2(w[r]);
                 ax += vv.x * ww.x + vv.y * ww.y;
                 ay += vv.x * ww.y - vv.y * ww.x;
             }
         } else {
-            for (int r = b + lane; r < e; r += 32) ax += w[r].x * w[r].x + w[r].y * w[r].y;
+            for (int r = b + lane; r < e; r += 32) {
+                const double2 ww = to_d2(w[r]);
+                ax += ww.x * ww.x + ww.y * ww.y;
+            }
         }
         ax = wred(ax);
         ay = wred(ay);
@@ -192,7 +197,8 @@ __device__ __forceinline__ void cycle_proj(const CycleArgs& a, int ncols, bool n
 }
 
 // coef[c] = sum over the blocks, the same order in every block
-__device__ __forceinline__ void cycle_reduce(const CycleArgs& a, int count, double2* coef) {
+template <typename VT>
+__device__ __forceinline__ void cycle_reduce(const CycleArgs<VT>& a, int count, double2* coef) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int c = wid; c < count; c += kCW) {
         const double2* p = a.part + (int64_t)c * gridDim.x;
@@ -210,8 +216,9 @@ __device__ __forceinline__ void cycle_reduce(const CycleArgs& a, int count, doub
 }
 
 // w -= sum_i coef[i] V_i on the block's rows, S lanes per row; the block's |w|^2 to npart, w to xn
-__device__ __forceinline__ void cycle_update(const CycleArgs& a, int ncols, int64_t r0, int nr, double2* w,
-                                             const double2* coef, double2* xn, double* red) {
+template <typename VT>
+__device__ __forceinline__ void cycle_update(const CycleArgs<VT>& a, int ncols, int64_t r0, int nr, VT* w,
+                                             const double2* coef, VT* xn, double* red) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int S = a.split, rl = 32 / S, s = lane / rl;
     double n2 = 0.0;
@@ -220,10 +227,10 @@ __device__ __forceinline__ void cycle_update(const CycleArgs& a, int ncols, int6
         const bool in = r < nr;
         double ax = 0.0, ay = 0.0;
         if (in) {
-            const double2* v = a.V + r0 + r;
+            const VT* v = a.V + r0 + r;
 #pragma unroll 4
             for (int i = s; i < ncols; i += S) {
-                const double2 c = coef[i], vv = v[(int64_t)i * a.N];
+                const double2 c = coef[i], vv = to_d2(v[(int64_t)i * a.N]);
                 ax += c.x * vv.x - c.y * vv.y;
                 ay += c.x * vv.y + c.y * vv.x;
             }
@@ -233,10 +240,12 @@ __device__ __forceinline__ void cycle_update(const CycleArgs& a, int ncols, int6
             ay += __shfl_xor_sync(kAll, ay, o);
         }
         if (in && s == 0) {
-            const double2 v = make_double2(w[r].x - ax, w[r].y - ay);
+            const double2 wv = to_d2(w[r]);
+            const VT v = from_d2<VT>(make_double2(wv.x - ax, wv.y - ay));
             w[r] = v;
             if (xn) xn[r0 + r] = v;
-            n2 += v.x * v.x + v.y * v.y;
+            const double2 back = to_d2(v);           // the norm of what is kept
+            n2 += back.x * back.x + back.y * back.y;
         }
     }
     n2 = wred(n2);
@@ -249,7 +258,8 @@ __device__ __forceinline__ void cycle_update(const CycleArgs& a, int ncols, int6
 }
 
 // |w|^2 over all blocks (every thread)
-__device__ __forceinline__ double cycle_norm(const CycleArgs& a, double* red) {
+template <typename VT>
+__device__ __forceinline__ double cycle_norm(const CycleArgs<VT>& a, double* red) {
     const int lane = threadIdx.x & 31;
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -264,23 +274,24 @@ __device__ __forceinline__ double cycle_norm(const CycleArgs& a, double* red) {
     return v;
 }
 
-template <int MAP>
-__global__ void __launch_bounds__(kCT, 1) k_lanczos_cycle(CycleArgs a) {
+template <typename VT, int MAP>
+__global__ void __launch_bounds__(kCT, 1) k_lanczos_cycle(CycleArgs<VT> a) {
     extern __shared__ double2 sm[];
-    double2* w = sm;                                 // [rows]
-    double2* coef = w + a.rows;                      // [kMaxCols + 1]
+    double2* coef = sm;                              // [kMaxCols + 1]
     double2* slot = coef + kMaxCols + 1;             // [(kMaxCols + 1) * chunks]
+    VT* w = reinterpret_cast<VT*>(slot + (kMaxCols + 1) * a.chunks);   // [rows]
     __shared__ double red[kCW];
     if (*(volatile int*)a.err) return;               // an earlier launch of the solve gave up
     const int64_t r0 = (int64_t)blockIdx.x * a.rows;
     const int nr = (int)max((int64_t)0, min((int64_t)a.rows, a.N - r0));
     unsigned target = 0;
     double s = 1.0;
-    const double2* x = a.V + (int64_t)a.j0 * a.N;
+    const VT* x = a.V + (int64_t)a.j0 * a.N;
     for (int j = a.j0; j < a.j1; ++j) {
         const int nc = j + 1;
-        double2* vn = a.V + (int64_t)nc * a.N;
-        double2* xn = MAP == CYCLE_NONE ? nullptr : a.xbuf + (int64_t)(j & 1) * a.N;
+        VT* vn = a.V + (int64_t)nc * a.N;
+        VT* xn = nullptr;
+        if constexpr (MAP != CYCLE_NONE) xn = a.xbuf + (int64_t)(j & 1) * a.N;
         if constexpr (MAP == CYCLE_NONE) {
             for (int r = threadIdx.x; r < nr; r += kCT) w[r] = vn[r0 + r];
         } else {
@@ -295,8 +306,7 @@ __global__ void __launch_bounds__(kCT, 1) k_lanczos_cycle(CycleArgs a) {
         cycle_update(a, nc, r0, nr, w, coef, xn, red);
         if (!grid_barrier(a.bar, target, a.err)) return;
         double after = cycle_norm(a, red);
-        // the second pass by k_decide's rule (vecops.cu)
-        if (after < 0.1 * before) {
+        if (after < a.keep * before) {
             cycle_proj(a, nc, false, r0, nr, w, slot);
             if (!grid_barrier(a.bar, target, a.err)) return;
             cycle_reduce(a, nc, coef);
@@ -307,7 +317,10 @@ __global__ void __launch_bounds__(kCT, 1) k_lanczos_cycle(CycleArgs a) {
         }
         const double b = sqrt(max(after, 0.0));
         s = b > 0.0 ? 1.0 / b : 0.0;
-        for (int r = threadIdx.x; r < nr; r += kCT) vn[r0 + r] = make_double2(w[r].x * s, w[r].y * s);
+        for (int r = threadIdx.x; r < nr; r += kCT) {
+            const double2 v = to_d2(w[r]);
+            vn[r0 + r] = from_d2<VT>(make_double2(v.x * s, v.y * s));
+        }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             a.alpha[j] = alpha;
             a.beta[j] = b;
@@ -336,39 +349,49 @@ int cycle_sms() {
     return s;
 }
 
-size_t cycle_smem(int rows, int chunks) {
-    return ((size_t)rows + (kMaxCols + 1) * (size_t)(1 + chunks)) * sizeof(double2);
+size_t cycle_smem(int rows, int chunks, size_t elem) {
+    return (kMaxCols + 1) * (size_t)(1 + chunks) * sizeof(double2) + (size_t)rows * elem;
 }
 
 }  // namespace
 
-// Rows per block and the split of a block's work; false where a block's part of w does not fit.
 // Small sectors take at least 32 rows a block (a barrier over few blocks is shorter).
-bool cycle_plan(int64_t N, CycleArgs& a, int& grid) {
+template <typename VT>
+bool cycle_plan(int64_t N, CycleArgs<VT>& a, int& grid) {
     const int sms = cycle_sms();
     if (N < 1 || sms < 1) return false;
     const int64_t rows = std::max<int64_t>(32, (N + sms - 1) / sms);
-    if (rows > (int64_t)(kMaxSmem / sizeof(double2))) return false;
+    if (rows > (int64_t)(kMaxSmem / sizeof(VT))) return false;
     a.N = N;
     a.rows = (int)rows;
     a.chunks = (int)std::min<int64_t>(kMaxChunks, std::max<int64_t>(1, rows / 128));
     a.split = rows <= 512 ? 4 : rows <= 2048 ? 2 : 1;
     grid = (int)((N + rows - 1) / rows);
-    return cycle_smem(a.rows, a.chunks) <= kMaxSmem;
+    return cycle_smem(a.rows, a.chunks, sizeof(VT)) <= kMaxSmem;
 }
 
-void launch_cycle(CycleArgs& a, int map, int grid, cudaStream_t st) {
-    const size_t smem = cycle_smem(a.rows, a.chunks);
+template <typename VT>
+void launch_cycle(CycleArgs<VT>& a, int map, int grid, cudaStream_t st) {
+    const size_t smem = cycle_smem(a.rows, a.chunks, sizeof(VT));
     void* args[] = {&a};
     auto go = [&](auto k) {
         // process-wide attribute: always the largest size, so concurrent callers never lower it
         MOMED_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
         MOMED_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(grid), dim3(kCT), args, smem, st));
     };
-    if (map == CYCLE_HITS) go(k_lanczos_cycle<CYCLE_HITS>);
-    else if (map == CYCLE_CSR) go(k_lanczos_cycle<CYCLE_CSR>);
-    else go(k_lanczos_cycle<CYCLE_NONE>);
+    if constexpr (std::is_same<VT, double2>::value) {
+        if (map == CYCLE_HITS) go(k_lanczos_cycle<double2, CYCLE_HITS>);
+        else if (map == CYCLE_CSR) go(k_lanczos_cycle<double2, CYCLE_CSR>);
+        else go(k_lanczos_cycle<double2, CYCLE_NONE>);
+    } else {
+        go(k_lanczos_cycle<float2, CYCLE_NONE>);
+    }
     note_launches(1);
 }
+
+template bool cycle_plan<double2>(int64_t, CycleArgs<double2>&, int&);
+template bool cycle_plan<float2>(int64_t, CycleArgs<float2>&, int&);
+template void launch_cycle<double2>(CycleArgs<double2>&, int, int, cudaStream_t);
+template void launch_cycle<float2>(CycleArgs<float2>&, int, int, cudaStream_t);
 
 }  // namespace momed

@@ -1,4 +1,4 @@
-// Cooperative kernel for the steps of an FP64 Lanczos cycle (cycle.cu).
+// Cooperative kernel for the steps of a single-vector Lanczos cycle (cycle.cu).
 #pragma once
 #include "vecops.cuh"
 
@@ -6,8 +6,9 @@ namespace momed {
 
 enum CycleMap : int { CYCLE_NONE = 0, CYCLE_HITS = 1, CYCLE_CSR = 2 };
 
-struct CycleArgs {
-    double2* V;                // basis, column i at V + i N
+// VT: the basis, double2 or float2 (FP32 vectors, FP64 sums; the map beside it only).
+template <typename VT> struct CycleArgs {
+    VT* V;                     // basis, column i at V + i N
     int64_t N;
     int j0, j1;                // steps [j0, j1); column j0 is normalised
     int rows, chunks, split;   // cycle_plan
@@ -15,6 +16,7 @@ struct CycleArgs {
     double* npart;             // [blocks]
     double2* xbuf;             // [2][N] vectors before their scaling (with the map inside)
     double *alpha, *beta;      // [m]
+    double keep;               // second Gram-Schmidt pass when less than this share of |w|^2 is left
     unsigned* bar;             // [2] zero between launches
     int* err;                  // set when a barrier gave up
     const int64_t* row_ptr;    // hit records or CSR
@@ -26,7 +28,45 @@ struct CycleArgs {
     const double2* val;
 };
 
-bool cycle_plan(int64_t N, CycleArgs& a, int& grid);
-void launch_cycle(CycleArgs& a, int map, int grid, cudaStream_t st);
+// Rows per block and the split of a block's work; false where a block's part of w does not fit.
+template <typename VT> bool cycle_plan(int64_t N, CycleArgs<VT>& a, int& grid);
+template <typename VT> void launch_cycle(CycleArgs<VT>& a, int map, int grid, cudaStream_t st);
+
+// The buffers of a solve's launches (partial sums, barrier) beside those the solver owns.
+template <typename VT> struct CycleBufs {
+    CycleArgs<VT> a{};
+    int grid = 0;
+    DevBuf<double2> part, xbuf;
+    DevBuf<double> npart;
+    DevBuf<unsigned> bar;
+    // false: the solver runs its separate kernels
+    bool prepare(int64_t N, bool with_map, double* alpha, double* beta, double keep, cudaStream_t st) {
+        if (!cycle_plan(N, a, grid)) return false;
+        part.resize((size_t)grid * (kMaxCols + 1));
+        npart.resize(grid);
+        bar.resize(3);                   // barrier, its exits, the error flag
+        MOMED_CUDA_TRY(cudaMemsetAsync(bar.p, 0, 3 * sizeof(unsigned), st));
+        if (with_map) xbuf.resize((size_t)2 * N);
+        a.part = part.p;
+        a.npart = npart.p;
+        a.xbuf = xbuf.p;
+        a.alpha = alpha;
+        a.beta = beta;
+        a.keep = keep;
+        a.bar = bar.p;
+        a.err = reinterpret_cast<int*>(bar.p + 2);
+        return true;
+    }
+    void steps(VT* V, int j0, int j1, int map, cudaStream_t st) {
+        a.V = V;
+        a.j0 = j0;
+        a.j1 = j1;
+        launch_cycle(a, map, grid, st);
+    }
+    // after a synchronisation of the copy of err: a barrier that gave up ends the solve
+    static void check(int err) {
+        if (err) throw Error{MOMED_ETIMEOUT, "Lanczos cycle: a grid barrier gave up"};
+    }
+};
 
 }  // namespace momed

@@ -114,11 +114,7 @@ struct Lanczos {
     std::vector<double> Uc;          // restart coefficients, alive until their copy has run
     // cooperative steps (cycle.cu): FP64 without per-launch timing
     int coop = -1;                   // CycleMap, -1: the separate kernels
-    int coop_grid = 0;
-    CycleArgs ca{};
-    DevBuf<double2> cpart, xbuf;
-    DevBuf<double> npart;
-    DevBuf<unsigned> bar;
+    CycleBufs<double2> cy;
 
     Lanczos(momed_handle* hh, int mm) : h(hh), N(hh->n), m(mm), st(hh->stream) {
         grid = vec_grid(N);
@@ -144,43 +140,28 @@ struct Lanczos {
         if (h->sparse.built) coop = CYCLE_CSR;
         else if (h->hcache.pair.built) coop = CYCLE_NONE;
         else if (h->hcache.full()) coop = CYCLE_HITS;
-        if (coop < 0 || !cycle_plan(N, ca, coop_grid)) {
+        if (coop < 0) return;
+        if (!cy.prepare(N, coop != CYCLE_NONE, alpha, beta, 0.1, st)) {     // k_decide's share
             coop = -1;
             return;
         }
-        cpart.resize((size_t)coop_grid * (kMaxCols + 1));
-        npart.resize(coop_grid);
-        bar.resize(3);                   // barrier, its exits, the error flag
-        MOMED_CUDA_TRY(cudaMemsetAsync(bar.p, 0, 3 * sizeof(unsigned), st));
-        if (coop != CYCLE_NONE) xbuf.resize((size_t)2 * N);
-        ca.part = cpart.p;
-        ca.npart = npart.p;
-        ca.xbuf = xbuf.p;
-        ca.alpha = alpha;
-        ca.beta = beta;
-        ca.bar = bar.p;
-        ca.err = reinterpret_cast<int*>(bar.p + 2);
+        CycleArgs<double2>& a = cy.a;
         if (coop == CYCLE_CSR) {
-            ca.row_ptr = h->sparse.row_ptr.p;
-            ca.col = h->sparse.col.p;
-            ca.val = h->sparse.val.p;
+            a.row_ptr = h->sparse.row_ptr.p;
+            a.col = h->sparse.col.p;
+            a.val = h->sparse.val.p;
         } else if (coop == CYCLE_HITS) {
             const HitCacheView hv = h->hcache.view();
-            ca.row_ptr = hv.row_ptr;
-            ca.hit = hv.hit;
-            ca.dg = hv.dg64;
-            ca.has_b = h->op.has_b ? 1 : 0;
-            ca.u = h->u;
-            ca.amp = hit_amplitudes_c128(h, st);
+            a.row_ptr = hv.row_ptr;
+            a.hit = hv.hit;
+            a.dg = hv.dg64;
+            a.has_b = h->op.has_b ? 1 : 0;
+            a.u = h->u;
+            a.amp = hit_amplitudes_c128(h, st);
         }
     }
     void coop_steps(int j0, int j1) {
-        if constexpr (std::is_same<VT, double2>::value) {
-            ca.V = V.p;
-            ca.j0 = j0;
-            ca.j1 = j1;
-            launch_cycle(ca, coop, coop_grid, st);
-        }
+        if constexpr (std::is_same<VT, double2>::value) cy.steps(V.p, j0, j1, coop, st);
     }
     // steps [j0, j1)
     void steps(int j0, int j1) {
@@ -195,9 +176,9 @@ struct Lanczos {
         int err = 0;
         std::vector<double> t((size_t)2 * m);
         MOMED_CUDA_TRY(cudaMemcpyAsync(t.data(), ab.p, t.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-        if (coop >= 0) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, ca.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (coop >= 0) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
         MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-        if (err) throw Error{MOMED_ETIMEOUT, "Lanczos cycle: a grid barrier gave up"};
+        CycleBufs<double2>::check(err);
         std::copy(t.begin(), t.begin() + m, ha);
         std::copy(t.begin() + m, t.end(), hb);
     }

@@ -229,6 +229,7 @@ void ensure_ready(momed_handle* h) {
 }
 
 thread_local cudaStream_t g_alloc_stream = nullptr;
+thread_local BlockCache* g_alloc_cache = nullptr;
 
 }  // namespace momed
 
@@ -237,7 +238,7 @@ namespace {
 template <typename F>
 int guarded(momed_handle* h, F&& f) {
     try {
-        AllocScope scope(h ? h->stream : g_alloc_stream);
+        AllocScope scope(h ? h->stream : g_alloc_stream, h ? &h->blocks : nullptr);
         if (h) {
             cudaError_t e = cudaSetDevice(h->device);
             if (e != cudaSuccess) throw Error{MOMED_ECUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e)};
@@ -270,6 +271,39 @@ void keep_pool_memory(int device) {
     done.push_back(device);
 }
 
+// Streams and events of closed handles, for the next ones on the device (creating and destroying a
+// stream took 0.2-0.6 ms of a 4 ms EDsolve call).  At most kIdle sets wait; they hold no memory.
+struct HandleParts {
+    int device;
+    cudaStream_t stream;
+    cudaEvent_t ev0, ev1;
+};
+constexpr size_t kIdle = 8;
+std::mutex g_parts_mu;
+std::vector<HandleParts>& idle_parts() {
+    static auto* v = new std::vector<HandleParts>();   // never destroyed: handles may close at exit
+    return *v;
+}
+bool take_parts(momed_handle* h) {
+    std::lock_guard<std::mutex> lk(g_parts_mu);
+    auto& v = idle_parts();
+    for (size_t i = 0; i < v.size(); ++i)
+        if (v[i].device == h->device) {
+            h->stream = v[i].stream;
+            h->ev0 = v[i].ev0;
+            h->ev1 = v[i].ev1;
+            v.erase(v.begin() + i);
+            return true;
+        }
+    return false;
+}
+bool keep_parts(const HandleParts& p) {
+    std::lock_guard<std::mutex> lk(g_parts_mu);
+    if (idle_parts().size() >= kIdle) return false;
+    idle_parts().push_back(p);
+    return true;
+}
+
 void after_basis_change(momed_handle* h) {
     scan_basis(h);
     h->index_dirty = true;
@@ -299,11 +333,13 @@ int momed_create(int device, momed_handle** out) {
     h->device = device;
     int rc = guarded(h, [&]() {
         keep_pool_memory(device);
-        MOMED_CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+        if (!take_parts(h)) {
+            MOMED_CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+            MOMED_CUDA_TRY(cudaEventCreate(&h->ev0));
+            MOMED_CUDA_TRY(cudaEventCreate(&h->ev1));
+        }
         h->own_stream = true;
         g_alloc_stream = h->stream;   // this call's scope (set before the stream existed)
-        MOMED_CUDA_TRY(cudaEventCreate(&h->ev0));
-        MOMED_CUDA_TRY(cudaEventCreate(&h->ev1));
         std::vector<uint32_t> b(33 * 33, 0);
         for (int n = 0; n <= 32; ++n)
             for (int k = 0; k <= n; ++k) {
@@ -334,22 +370,29 @@ int momed_create(int device, momed_handle** out) {
 int momed_destroy(momed_handle* h) {
     if (!h) return MOMED_OK;
     cudaSetDevice(h->device);
-    if (h->stream) cudaStreamSynchronize(h->stream);
+    cudaError_t se = h->stream ? cudaStreamSynchronize(h->stream) : cudaErrorInvalidResourceHandle;
     for (cudaEvent_t e : h->prof_ev) cudaEventDestroy(e);
-    if (h->ev0) cudaEventDestroy(h->ev0);
-    if (h->ev1) cudaEventDestroy(h->ev1);
     cudaStream_t hs = h->stream;
     const bool own = h->own_stream;
+    const HandleParts parts{h->device, hs, h->ev0, h->ev1};
     {
         AllocScope scope(hs);
+        h->blocks.flush(hs);
         delete h;   // releases every DevBuf, ordered on the handle's stream
     }
-    cudaStreamSynchronize(hs);
-    if (own && hs) cudaStreamDestroy(hs);
+    if (se == cudaSuccess) se = cudaStreamSynchronize(hs);
+    const bool whole = own && hs && parts.ev0 && parts.ev1 && se == cudaSuccess;
+    if (!whole || !keep_parts(parts)) {
+        if (parts.ev0) cudaEventDestroy(parts.ev0);
+        if (parts.ev1) cudaEventDestroy(parts.ev1);
+        if (own && hs) cudaStreamDestroy(hs);
+    }
     cudaMemPool_t pool;
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
-        cudaMemPoolTrimTo(pool, 0);   // return blocks no other handle is using
+        // return blocks no other handle is using, up to what small solves allocate: programs that
+        // open a handle per sector (EDsolve) otherwise map that memory again each time
+        cudaMemPoolTrimTo(pool, kSmallBytes);
     return MOMED_OK;
 }
 
@@ -372,6 +415,8 @@ int momed_set_stream(momed_handle* h, void* s) {
 int momed_set_hbm_budget(momed_handle* h, int64_t bytes) {
     if (!h || bytes < 0) return MOMED_EINVAL;
     h->hbm_budget = bytes;
+    h->blocks.on = bytes == 0;
+    if (bytes > 0) h->blocks.flush(h->stream);
     return MOMED_OK;
 }
 

@@ -382,6 +382,20 @@ int sms() {
     return s;
 }
 
+// f(0) .. f(n - 1) on at most eight threads, this one among them (a thread per right-hand side took
+// longer to start than its small eigenproblem)
+template <typename F>
+void host_parallel(int n, F&& f) {
+    std::atomic<int> next{0};
+    auto work = [&]() {
+        for (int i = next.fetch_add(1); i < n; i = next.fetch_add(1)) f(i);
+    };
+    std::vector<std::future<void>> fs;
+    for (int t = 1; t < std::min(n, 8); ++t) fs.push_back(std::async(std::launch::async, work));
+    work();
+    for (auto& x : fs) x.get();
+}
+
 template <typename VT> struct BlockMv;
 template <> struct BlockMv<float2> {
     // u0: the host's copy of u[0]; one right-hand side runs the single-vector map over the pair tables
@@ -634,8 +648,7 @@ struct BlockLanczos {
     void recombine(const std::vector<double>& Uh, int keep) {
         V2.resize((size_t)(m + 1) * N * NB);
         combine<VT>(Uh, keep, V2.p, m, m);
-        std::swap(V.p, V2.p);
-        std::swap(V.n, V2.n);
+        V.swap(V2);
     }
 
     struct Out {
@@ -726,11 +739,7 @@ struct BlockLanczos {
                     if (hb[(size_t)r * m + j] <= 1e-13 * sc) out.broken[r] = 1;
                 if (out.broken[r]) nconv[r] = nev;   // finished separately by the single-vector solver
             };
-            {
-                std::vector<std::future<void>> fs;
-                for (int r = 0; r < NB; ++r) fs.push_back(std::async(std::launch::async, solve_r, r));
-                for (auto& f : fs) f.get();
-            }
+            host_parallel(NB, solve_r);
             int minconv = nev;
             for (int r = 0; r < nu; ++r) minconv = std::min(minconv, nconv[r]);
             if (minconv >= nev || restarts >= maxiter) {
@@ -1134,31 +1143,25 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
         std::vector<double2> Yh((size_t)NB * k1 * k1, make_double2(0.0, 0.0));
         for (int q = 0; q < NB; ++q)
             for (int i = 0; i < k1; ++i) Yh[((size_t)q * k1 + i) * k1 + i] = make_double2(1.0, 0.0);
-        {
-            std::vector<std::future<void>> fs;
-            for (int q = 0; q < nu; ++q) {
-                if (broken[q]) continue;
-                fs.push_back(std::async(std::launch::async, [&, q]() {
-                    std::vector<double> t;
-                    std::vector<std::complex<double>> Y;
-                    if (!gen_herm_eig(k1, G[q], S[q], t, Y)) { broken[q] = 1; return; }
-                    th[q] = t;
-                    for (int i = 0; i < k1; ++i)
-                        for (int a = 0; a < k1; ++a) {
-                            auto y = Y[(size_t)i * k1 + a];
-                            Yh[((size_t)q * k1 + i) * k1 + a] = make_double2(y.real(), y.imag());
-                        }
-                }));
-            }
-            for (auto& f : fs) f.get();
-        }
+        host_parallel(nu, [&](int q) {
+            if (broken[q]) return;
+            std::vector<double> t;
+            std::vector<std::complex<double>> Y;
+            if (!gen_herm_eig(k1, G[q], S[q], t, Y)) { broken[q] = 1; return; }
+            th[q] = t;
+            for (int i = 0; i < k1; ++i)
+                for (int a = 0; a < k1; ++a) {
+                    auto y = Y[(size_t)i * k1 + a];
+                    Yh[((size_t)q * k1 + i) * k1 + a] = make_double2(y.real(), y.imag());
+                }
+        });
         DevBuf<double2> Yd;
         Yd.resize(Yh.size());
         MOMED_CUDA_TRY(cudaMemcpyAsync(Yd.p, Yh.data(), Yh.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
         k_bcombine_c<NB><<<eg, 256, 0, st>>>(Xb.p, N, k1, Yd.p, Sb.p);
-        std::swap(Xb.p, Sb.p);
+        Xb.swap(Sb);
         k_bcombine_c<NB><<<eg, 256, 0, st>>>(Wb.p, N, k1, Yd.p, Sb.p);
-        std::swap(Wb.p, Sb.p);
+        Wb.swap(Sb);
         note_launches(2);
         MOMED_CUDA_TRY(cudaGetLastError());
         MOMED_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1374,10 +1377,8 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                 std::vector<std::vector<double>> tq(NB);
                 std::vector<int> ok_rr(NB, 0);
                 {
-                    std::vector<std::future<void>> fs;
-                    for (int q = 0; q < nu; ++q) {
-                        if (broken[q] || failed[q]) continue;
-                        fs.push_back(std::async(std::launch::async, [&, q]() {
+                    host_parallel(nu, [&](int q) {
+                            if (broken[q] || failed[q]) return;
                             double tmax = 0.0;
                             for (int i = 0; i < k1; ++i) tmax = std::max(tmax, std::fabs(th[q][i]));
                             for (int j = 0; j < p; ++j) {
@@ -1425,9 +1426,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                             }
                             tq[q] = t;
                             ok_rr[q] = 1;
-                        }));
-                    }
-                    for (auto& f : fs) f.get();
+                    });
                 }
                 for (int q = 0; q < NB; ++q) {
                     if (ok_rr[q]) continue;
@@ -1446,8 +1445,8 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                 k_bcombine_xq<NB><<<xg, kT, 0, st>>>(Wb.p, k1, Xb.p, k1, LR.col(k1), p + 1, N, Y2d.p, k1, W2.p);
                 note_launches(2);
                 MOMED_CUDA_TRY(cudaGetLastError());
-                std::swap(Xb.p, Sb.p);
-                std::swap(Wb.p, W2.p);
+                Xb.swap(Sb);
+                Wb.swap(W2);
                 for (int q = 0; q < nu; ++q)
                     if (ok_rr[q]) {
                         for (int i = 0; i < k1; ++i) th[q][i] = tq[q][i];

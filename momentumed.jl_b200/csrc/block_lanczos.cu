@@ -694,8 +694,7 @@ struct BlockKrylov {
             combine_blocked(Y, m, nk, Q2.p);
             MOMED_CUDA_TRY(cudaMemcpyAsync(Q2.p + (size_t)nkb * N * B, blk(mb), (size_t)N * B * sizeof(VT),
                                            cudaMemcpyDeviceToDevice, st));
-            std::swap(Q.p, Q2.p);
-            std::swap(Q.n, Q2.n);
+            Q.swap(Q2);
             kept_theta.assign(th.begin(), th.begin() + nk);
             S.assign((size_t)B * nk, 0.0);
             for (int a = 0; a < B; ++a)

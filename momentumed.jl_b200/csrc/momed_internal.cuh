@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/momed.h"
@@ -46,10 +47,69 @@ inline std::string base_name(const char* path) {
 // (cudaMallocAsync / cudaFreeAsync from the device's default memory pool), so freeing a solve's
 // buffers does not synchronise the device and solves on other streams keep running.
 extern thread_local cudaStream_t g_alloc_stream;
+
+// Large blocks that a handle's buffers gave back, kept for its next solve.  A solve frees and
+// allocates gigabytes; from the device's pool a block freed on one stream and taken on another
+// (several handles in turn) is often not reusable yet, and the pool maps new memory instead
+// (measured: 30-70 ms of a 3x10 solve or a 32-parameter sweep, once 1.1 s).  All of a handle's
+// buffers are ordered on its one stream, so its own blocks need no event.  Held at most kMaxHeld
+// bytes; given back to the pool when an allocation is refused, when a budget is set and with the
+// handle.  Off for handles with an HBM budget and for serving slots, which account for every byte.
+struct BlockCache {
+    static constexpr size_t kMinBlock = size_t(1) << 20;
+    static constexpr size_t kMaxHeld = size_t(16) << 30;
+    struct Block { void* p; size_t bytes; };
+    std::vector<Block> blocks;             // oldest first
+    size_t held = 0;
+    bool on = true;
+    // a block of at least `bytes`, at most a quarter larger; null: none
+    void* take(size_t bytes, size_t& got) {
+        size_t best = blocks.size();
+        for (size_t i = 0; i < blocks.size(); ++i)
+            if (blocks[i].bytes >= bytes && blocks[i].bytes <= bytes + bytes / 4 &&
+                (best == blocks.size() || blocks[i].bytes < blocks[best].bytes))
+                best = i;
+        if (best == blocks.size()) return nullptr;
+        void* p = blocks[best].p;
+        got = blocks[best].bytes;
+        held -= got;
+        blocks.erase(blocks.begin() + best);
+        return p;
+    }
+    bool put(void* p, size_t bytes, cudaStream_t st) noexcept {
+        if (!on || bytes < kMinBlock || bytes > kMaxHeld) return false;
+        try {
+            blocks.push_back({p, bytes});
+        } catch (...) {
+            return false;
+        }
+        held += bytes;
+        while (held > kMaxHeld) {
+            cudaFreeAsync(blocks.front().p, st);
+            held -= blocks.front().bytes;
+            blocks.erase(blocks.begin());
+        }
+        return true;
+    }
+    void flush(cudaStream_t st) noexcept {
+        for (const Block& b : blocks) cudaFreeAsync(b.p, st);
+        blocks.clear();
+        held = 0;
+    }
+};
+extern thread_local BlockCache* g_alloc_cache;
+
 struct AllocScope {
     cudaStream_t prev;
-    explicit AllocScope(cudaStream_t s) : prev(g_alloc_stream) { g_alloc_stream = s; }
-    ~AllocScope() { g_alloc_stream = prev; }
+    BlockCache* prev_cache;
+    explicit AllocScope(cudaStream_t s, BlockCache* c = nullptr) : prev(g_alloc_stream), prev_cache(g_alloc_cache) {
+        g_alloc_stream = s;
+        g_alloc_cache = c;
+    }
+    ~AllocScope() {
+        g_alloc_stream = prev;
+        g_alloc_cache = prev_cache;
+    }
     AllocScope(const AllocScope&) = delete;
     AllocScope& operator=(const AllocScope&) = delete;
 };
@@ -59,25 +119,47 @@ template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
+    size_t cap = 0;                        // bytes of the block behind it
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+    DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), cap(o.cap) { o.p = nullptr; o.n = o.cap = 0; }
     DevBuf& operator=(DevBuf&& o) noexcept {
-        if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+        if (this != &o) { release(); p = o.p; n = o.n; cap = o.cap; o.p = nullptr; o.n = o.cap = 0; }
         return *this;
     }
     ~DevBuf() { release(); }
     void release() {
-        if (p) cudaFreeAsync(p, g_alloc_stream);
+        if (p && !(g_alloc_cache && g_alloc_cache->put(p, cap, g_alloc_stream))) cudaFreeAsync(p, g_alloc_stream);
         p = nullptr;
-        n = 0;
+        n = cap = 0;
+    }
+    // the two exchange their blocks
+    void swap(DevBuf& o) noexcept {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+        std::swap(cap, o.cap);
     }
     void resize(size_t count) {
         if (count <= n && p) return;
         release();
         if (count == 0) return;
-        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), count * sizeof(T), g_alloc_stream);
+        const size_t bytes = count * sizeof(T);
+        BlockCache* const c = g_alloc_cache;
+        if (c && c->on && bytes >= BlockCache::kMinBlock) {
+            p = static_cast<T*>(c->take(bytes, cap));
+            if (p) {
+                n = count;
+                return;
+            }
+        }
+        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, g_alloc_stream);
+        if (e != cudaSuccess && c && c->held > 0) {        // once more with the kept blocks back in the pool
+            cudaGetLastError();
+            c->flush(g_alloc_stream);
+            cudaStreamSynchronize(g_alloc_stream);
+            e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, g_alloc_stream);
+        }
         if (e != cudaSuccess) {
             p = nullptr;
             cudaGetLastError();
@@ -85,6 +167,7 @@ struct DevBuf {
                                           " bytes failed: " + cudaGetErrorString(e)};
         }
         n = count;
+        cap = bytes;
     }
     size_t bytes() const { return n * sizeof(T); }
 };
@@ -338,6 +421,7 @@ struct momed_handle {
     bool own_stream = false;
     std::string last_error;
     int64_t hbm_budget = 0;
+    momed::BlockCache blocks;              // declared before the buffers that give back to it
 
     int64_t n = 0;                         // basis size
     momed::DevBuf<uint64_t> basis;
@@ -390,6 +474,12 @@ namespace momed {
 
 // binomial table C(n, k), n, k in [0, 32], on the device (built once per process per device)
 const uint32_t* device_binomials();
+
+// hitcache.cu: whether bytes fit the share of the free device memory (the handle's kept blocks count
+// as free).  Up to kSmallBytes, and up to what the handle has kept, nothing is asked: cudaMemGetInfo
+// took 0.1 to 14 ms
+constexpr int64_t kSmallBytes = 64 << 20;
+bool fits_free(const momed_handle* h, int64_t bytes, double share);
 
 // index.cu
 void build_index(momed_handle* h);

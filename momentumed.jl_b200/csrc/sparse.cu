@@ -333,6 +333,12 @@ int spmv_grid(int64_t rows) {
 // column, FP64 value and its FP32 rounding; a parametrised operator also keeps A and B in c64
 int64_t sparse_bytes_per_entry(bool pair) { return 4 + 16 + 8 + (pair ? 16 : 0); }
 
+static void require_room(const momed_handle* h, int64_t need) {
+    if ((h->hbm_budget > 0 && need > h->hbm_budget) || !fits_free(h, need, 0.9))
+        throw Error{MOMED_ENOMEM, "sparse method: the matrix needs " + std::to_string(need) +
+                                     " bytes, more than is available"};
+}
+
 void build_sparse(momed_handle* h, double u) {
     SparseMatrix& sp = h->sparse;
     sp.release();
@@ -360,13 +366,7 @@ void build_sparse(momed_handle* h, double u) {
     // admission: row pointers plus column, FP64 value and FP32 value per entry
     const bool hb = h->op.has_b;
     const int64_t need = (n + 1) * 8 + nnz * sparse_bytes_per_entry(hb);
-    size_t free_b = 0, total_b = 0;
-    MOMED_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    int64_t limit = (int64_t)(0.9 * (double)free_b);
-    if (h->hbm_budget > 0) limit = std::min<int64_t>(limit, h->hbm_budget);
-    if (need > limit)
-        throw Error{MOMED_ENOMEM, "sparse method: the matrix needs " + std::to_string(need) + " bytes, " +
-                                     std::to_string(limit) + " available"};
+    require_room(h, need);
 
     sp.row_ptr.resize(n + 1);
     sp.col.resize(std::max<int64_t>(nnz, 1));
@@ -412,13 +412,7 @@ void upload_sparse(momed_handle* h, int64_t n, const int64_t* row_ptr, const int
     cudaStream_t st = h->stream;
     const int64_t nnz = row_ptr[n];
     const int64_t need = (n + 1) * 8 + nnz * sparse_bytes_per_entry(false);
-    size_t free_b = 0, total_b = 0;
-    MOMED_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    int64_t limit = (int64_t)(0.9 * (double)free_b);
-    if (h->hbm_budget > 0) limit = std::min<int64_t>(limit, h->hbm_budget);
-    if (need > limit)
-        throw Error{MOMED_ENOMEM, "sparse method: the matrix needs " + std::to_string(need) + " bytes, " +
-                                     std::to_string(limit) + " available"};
+    require_room(h, need);
     sp.row_ptr.resize(n + 1);
     sp.col.resize(std::max<int64_t>(nnz, 1));
     sp.val.resize(std::max<int64_t>(nnz, 1));

@@ -18,8 +18,16 @@ namespace momed {
 
 namespace {
 
+// sqrt(a^2 + b^2); std::hypot, which guards the whole range and costs a third of a small
+// eigenproblem, only where the squares would leave the normal range
+inline double pyth(double a, double b) {
+    const double s = a * a + b * b;
+    return s > 1e-280 && s < 1e280 ? std::sqrt(s) : std::hypot(a, b);
+}
+
 // Implicitly shifted QL on the symmetric tridiagonal (d, e), e[i] coupling d[i] and d[i+1];
-// the rotations are applied to the columns of Q (row-major n x n).  d ends as the eigenvalues.
+// the rotations are applied to the rows of Q (row-major n x n: row i is the i-th vector, so a
+// rotation runs over contiguous memory).  d ends as the eigenvalues.
 void tridiag_ql(int n, std::vector<double>& d, std::vector<double>& e, double* Q) {
     // implicit QL on (d, e); e[i] couples d[i] and d[i+1]
     const double eps = std::numeric_limits<double>::epsilon();
@@ -33,14 +41,14 @@ void tridiag_ql(int n, std::vector<double>& d, std::vector<double>& e, double* Q
             if (m == l) break;
             // shift from the leading 2x2 block
             double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-            double r = std::hypot(g, 1.0);
+            double r = pyth(g, 1.0);
             g = d[m] - d[l] + e[l] / (g + (g >= 0 ? r : -r));
             double s = 1.0, c = 1.0, pshift = 0.0;
             int i;
             bool deflated = false;
             for (i = m - 1; i >= l; --i) {
                 double f = s * e[i], b = c * e[i];
-                r = std::hypot(f, g);
+                r = pyth(f, g);
                 e[i + 1] = r;
                 if (r == 0.0) {
                     d[i + 1] -= pshift;
@@ -55,10 +63,12 @@ void tridiag_ql(int n, std::vector<double>& d, std::vector<double>& e, double* Q
                 pshift = s * r;
                 d[i + 1] = g + pshift;
                 g = c * r - b;
+                double* qa = Q + (size_t)i * n;
+                double* qb = qa + n;
                 for (int k = 0; k < n; ++k) {
-                    double qi1 = Q[(size_t)k * n + i + 1], qi = Q[(size_t)k * n + i];
-                    Q[(size_t)k * n + i + 1] = s * qi + c * qi1;
-                    Q[(size_t)k * n + i] = c * qi - s * qi1;
+                    const double qi1 = qb[k], qi = qa[k];
+                    qb[k] = s * qi + c * qi1;
+                    qa[k] = c * qi - s * qi1;
                 }
             }
             if (deflated) continue;
@@ -75,7 +85,7 @@ void tridiag_ql(int n, std::vector<double>& d, std::vector<double>& e, double* Q
 void symeig(int n, double* A, double* w, double* V) {
     if (n <= 0) return;
     // Q accumulates the Householder reflections; A is reduced in place.
-    std::vector<double> Q((size_t)n * n, 0.0), v(n), p(n), q(n);
+    std::vector<double> Q((size_t)n * n, 0.0), v(n), p(n), q(n), t(n);
     for (int i = 0; i < n; ++i) Q[(size_t)i * n + i] = 1.0;
     auto a = [&](int r, int c) -> double& { return A[(size_t)r * n + c]; };
 
@@ -95,25 +105,36 @@ void symeig(int n, double* A, double* w, double* V) {
         double inv = 1.0 / std::sqrt(vnorm2);
         for (int i = k + 1; i < n; ++i) v[i] *= inv;
         // trailing block: B <- (I - 2vv^T) B (I - 2vv^T) = B - 2 v q^T - 2 q v^T
-        for (int i = k + 1; i < n; ++i) {
-            double s = 0.0;
-            for (int j = k + 1; j < n; ++j) s += a(i, j) * v[j];
-            p[i] = s;
+        // p = B v by the rows of the symmetric B (each p[i] sums over j in order)
+        std::fill(p.begin() + k + 1, p.end(), 0.0);
+        for (int j = k + 1; j < n; ++j) {
+            const double* row = A + (size_t)j * n;
+            const double vj = v[j];
+            for (int i = k + 1; i < n; ++i) p[i] += row[i] * vj;
         }
         double K = 0.0;
         for (int i = k + 1; i < n; ++i) K += v[i] * p[i];
         for (int i = k + 1; i < n; ++i) q[i] = p[i] - K * v[i];
-        for (int i = k + 1; i < n; ++i)
-            for (int j = k + 1; j < n; ++j) a(i, j) -= 2.0 * (v[i] * q[j] + q[i] * v[j]);
+        for (int i = k + 1; i < n; ++i) {
+            double* row = A + (size_t)i * n;
+            const double vi = v[i], qi = q[i];
+            for (int j = k + 1; j < n; ++j) row[j] -= 2.0 * (vi * q[j] + qi * v[j]);
+        }
         a(k + 1, k) = alpha;
         a(k, k + 1) = alpha;
         for (int i = k + 2; i < n; ++i) { a(i, k) = 0.0; a(k, i) = 0.0; }
-        // Q <- Q (I - 2 v v^T)
-        for (int r = 0; r < n; ++r) {
-            double s = 0.0;
-            for (int j = k + 1; j < n; ++j) s += Q[(size_t)r * n + j] * v[j];
-            s *= 2.0;
-            for (int j = k + 1; j < n; ++j) Q[(size_t)r * n + j] -= s * v[j];
+        // Q <- (I - 2 v v^T) Q (the factor is kept transposed): t = v^T Q, row j loses 2 v_j t
+        std::fill(t.begin(), t.end(), 0.0);
+        for (int j = k + 1; j < n; ++j) {
+            const double* row = Q.data() + (size_t)j * n;
+            const double vj = v[j];
+            for (int r = 0; r < n; ++r) t[r] += row[r] * vj;
+        }
+        for (int r = 0; r < n; ++r) t[r] *= 2.0;
+        for (int j = k + 1; j < n; ++j) {
+            double* row = Q.data() + (size_t)j * n;
+            const double vj = v[j];
+            for (int r = 0; r < n; ++r) row[r] -= t[r] * vj;
         }
     }
 
@@ -128,7 +149,7 @@ void symeig(int n, double* A, double* w, double* V) {
     std::sort(ord.begin(), ord.end(), [&](int x, int y) { return d[x] < d[y]; });
     for (int c = 0; c < n; ++c) {
         w[c] = d[ord[c]];
-        for (int r = 0; r < n; ++r) V[(size_t)r * n + c] = Q[(size_t)r * n + ord[c]];
+        for (int r = 0; r < n; ++r) V[(size_t)r * n + c] = Q[(size_t)ord[c] * n + r];
     }
 }
 
@@ -202,7 +223,7 @@ void herm_eig(int n, std::complex<double>* A, double* w, std::complex<double>* Z
         w[c] = d[ord[c]];
         for (int r = 0; r < n; ++r) {
             cd s = 0.0;
-            for (int j = 0; j < n; ++j) s += Q[(size_t)r * n + j] * delta[j] * P[(size_t)j * n + ord[c]];
+            for (int j = 0; j < n; ++j) s += Q[(size_t)r * n + j] * delta[j] * P[(size_t)ord[c] * n + j];   // P kept transposed
             Z[(size_t)r * n + c] = s;
         }
     }

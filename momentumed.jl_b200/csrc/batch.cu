@@ -23,7 +23,7 @@
 #include <thread>
 #include <type_traits>
 
-#include "cycle.cuh"
+#include "blockstep.cuh"
 
 namespace momed {
 
@@ -41,37 +41,6 @@ template <int NB> __host__ __device__ constexpr int rows_tile() { return kTileEl
 constexpr double kEigTarget = 1e-11;
 // Anchored refinement cycles of the mixed-precision batch before the FP64 block Lanczos takes over.
 constexpr int kRefineCycles = 6;
-
-__device__ __forceinline__ double2 to2(double2 v) { return v; }
-__device__ __forceinline__ double2 to2(float2 v) { return make_double2(v.x, v.y); }
-template <typename VT> __device__ __forceinline__ VT fr2(double2 v);
-template <> __device__ __forceinline__ double2 fr2<double2>(double2 v) { return v; }
-template <> __device__ __forceinline__ float2 fr2<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
-
-// 16-byte packets of a block vector: two c64 values (adjacent right-hand sides of one row) when
-// NB is even, else one value.
-template <typename VT, int NB> struct Pack {
-    static constexpr int E = 1;
-    using T = VT;
-    static __device__ __forceinline__ void get(const T& p, double2* v) { v[0] = to2(p); }
-    static __device__ __forceinline__ T put(const double2* v) { return fr2<VT>(v[0]); }
-};
-template <int NB> struct PackF2 {
-    static constexpr int E = 2;
-    using T = float4;
-    static __device__ __forceinline__ void get(const float4& p, double2* v) {
-        v[0] = make_double2(p.x, p.y);
-        v[1] = make_double2(p.z, p.w);
-    }
-    static __device__ __forceinline__ float4 put(const double2* v) {
-        return make_float4((float)v[0].x, (float)v[0].y, (float)v[1].x, (float)v[1].y);
-    }
-};
-template <> struct Pack<float2, 2> : PackF2<2> {};
-template <> struct Pack<float2, 4> : PackF2<4> {};
-template <> struct Pack<float2, 8> : PackF2<8> {};
-template <> struct Pack<float2, 16> : PackF2<16> {};
-template <> struct Pack<float2, 32> : PackF2<32> {};
 
 // partial[b][i][r] (i <= ncols: column ncols holds |w_r|^2).  Grid: x = row blocks, y = groups
 // of 8 columns; warp w of group g owns column 8g + w over the block's rows, reading 16-byte
@@ -107,7 +76,7 @@ k_bproj(const VT* __restrict__ V, int64_t N, int ncols, const WT* __restrict__ W
             P::get(col[t * PR + rp], v);
 #pragma unroll
             for (int q = 0; q < E; ++q) {
-                const double2 w = to2(__ldg(wr + t * NB + q));
+                const double2 w = to_d2(__ldg(wr + t * NB + q));
                 ax[q] += v[q].x * w.x + v[q].y * w.y;
                 ay[q] += v[q].x * w.y - v[q].y * w.x;
                 if (norm) wn2[q] += w.x * w.x + w.y * w.y;
@@ -117,7 +86,7 @@ k_bproj(const VT* __restrict__ V, int64_t N, int ncols, const WT* __restrict__ W
         for (int64_t t = r0 + rs; t < r1; t += RS) {
 #pragma unroll
             for (int q = 0; q < E; ++q) {
-                const double2 w = to2(__ldg(wr + t * NB + q));
+                const double2 w = to_d2(__ldg(wr + t * NB + q));
                 wn2[q] += w.x * w.x + w.y * w.y;
             }
         }
@@ -276,8 +245,8 @@ __global__ void k_bscale(VT* W, int64_t N, const double* scal) {
     const int64_t total = N * NB;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
         double s = scal[e % NB];
-        double2 v = to2(W[e]);
-        W[e] = fr2<VT>(make_double2(v.x * s, v.y * s));
+        double2 v = to_d2(W[e]);
+        W[e] = from_d2<VT>(make_double2(v.x * s, v.y * s));
     }
 }
 
@@ -291,7 +260,7 @@ __global__ void k_brandom(VT* v, int64_t total, uint64_t seed) {
         };
         double a = (double)(mix(seed + (2 * (uint64_t)e + 1) * 0x9E3779B97F4A7C15ULL) >> 11) * (1.0 / 9007199254740992.0);
         double b = (double)(mix(seed + (2 * (uint64_t)e + 2) * 0x9E3779B97F4A7C15ULL) >> 11) * (1.0 / 9007199254740992.0);
-        v[e] = fr2<VT>(make_double2(a, b));
+        v[e] = from_d2<VT>(make_double2(a, b));
     }
 }
 
@@ -343,13 +312,13 @@ k_bcombine(const VIN* __restrict__ V, int64_t N, int m, const double* __restrict
 #pragma unroll
                 for (int k = 0; k < OC; ++k)
                     if (c0 + k < nout)
-                        out[(int64_t)(c0 + k) * stride + off[j]] = fr2<VOUT>(make_double2((double)ax[j][k], (double)ay[j][k]));
+                        out[(int64_t)(c0 + k) * stride + off[j]] = from_d2<VOUT>(make_double2((double)ax[j][k], (double)ay[j][k]));
             }
         }
         if (copy_col >= 0) {
 #pragma unroll
             for (int j = 0; j < RPT; ++j)
-                if (ok[j]) out[(int64_t)nout * stride + off[j]] = fr2<VOUT>(to2(V[(int64_t)copy_col * stride + off[j]]));
+                if (ok[j]) out[(int64_t)nout * stride + off[j]] = from_d2<VOUT>(to_d2(V[(int64_t)copy_col * stride + off[j]]));
         }
     }
 }
@@ -473,6 +442,11 @@ struct BlockLanczos {
     // instead of the map and eight kernels, and needs no graph.
     bool coop = false;
     CycleBufs<VT> cy;
+    // Otherwise the step beside the block map is one cooperative launch too (blockstep.cu: 364 us against
+    // 418 on 173.6k states x 32, 21 against 34 on 5.5k x 16); the separate kernels, and the graphs that
+    // replay them, stay for per-launch timing and MOMED_COOP=0.
+    bool coopb = false;
+    BlockStepBufs<VT> bs;
 
     ~BlockLanczos() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
@@ -523,7 +497,8 @@ struct BlockLanczos {
             use_graphs = !(e && e[0] == '0') && !hh->prof;   // per-launch timing needs eager launches
         }
         const char* ce = std::getenv("MOMED_COOP");
-        const bool want_coop = NB == 1 && !(ce && ce[0] == '0') && !hh->prof && !hh->sparse.built && hh->hcache.pair.built;
+        const bool any_coop = !(ce && ce[0] == '0') && !hh->prof;
+        const bool want_coop = NB == 1 && any_coop && !hh->sparse.built && hh->hcache.pair.built;
         {   // kernel attributes are set before any capture
             constexpr size_t smem_max = (size_t)kMaxCols * NB * sizeof(double2);
             if (smem_max > 48 * 1024)
@@ -546,6 +521,9 @@ struct BlockLanczos {
         any.resize(1);
         if (want_coop && cy.prepare(N, false, alpha.p, beta.p, dgks, st)) {
             coop = true;
+            use_graphs = false;
+        } else if (any_coop && bs.prepare(N, NB, m, alpha.p, beta.p, st)) {
+            coopb = true;
             use_graphs = false;
         }
         ud.resize(NB);
@@ -613,6 +591,10 @@ struct BlockLanczos {
         if (coop) {
             cy.a.keep = dgks;
             cy.steps(V.p, j, j + 1, CYCLE_NONE, st);
+            return;
+        }
+        if (coopb) {
+            bs.step(V.p, j, dgks, st);
             return;
         }
         const int nc = j + 1;
@@ -697,7 +679,8 @@ struct BlockLanczos {
             MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
             MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
             int err = 0;
-            if (coop) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            if (coop || coopb)
+                MOMED_CUDA_TRY(cudaMemcpyAsync(&err, coop ? cy.a.err : bs.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
             MOMED_CUDA_TRY(cudaStreamSynchronize(st));
             CycleBufs<VT>::check(err);
             // per right-hand side projected eigenproblems, in parallel on the host
@@ -858,7 +841,7 @@ __global__ void k_bresid_sum(const double2* __restrict__ W, const double2* __res
             sx += c * (w.x - t * x.x);
             sy += c * (w.y - t * x.y);
         }
-        out[e] = fr2<VT>(make_double2(sx, sy));
+        out[e] = from_d2<VT>(make_double2(sx, sy));
     }
 }
 
@@ -866,7 +849,7 @@ __global__ void k_bresid_sum(const double2* __restrict__ W, const double2* __res
 template <typename VT>
 __global__ void k_bto(const double2* __restrict__ X, int64_t total, VT* __restrict__ out) {
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x)
-        out[e] = fr2<VT>(X[e]);
+        out[e] = from_d2<VT>(X[e]);
 }
 
 // out[i][n][r] = sum_{a<kx} Y[i][a][r] X[a][n][r] + sum_{b<kz} Y[i][kx+b][r] Z[b][n][r]

@@ -38,49 +38,12 @@ constexpr int kCW = kCT / 32;
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kMaxChunks = 8;          // row chunks of a block's projections
 constexpr size_t kMaxSmem = 200 * 1024;
-constexpr uint64_t kWaitNs = 2000000000ull;   // a barrier gives up after two seconds
 
 __device__ __forceinline__ double wred(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kAll, v, o);
     return v;
 }
-__device__ __forceinline__ uint64_t now_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-
-// All blocks of the cooperative launch arrive; what they wrote before is visible after.  False (for
-// every thread of the block) when the wait ran out: the kernel then returns and the host reads err.
-__device__ bool grid_barrier(unsigned* bar, unsigned& target, int* err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (gridDim.x == 1) return true;
-    if (threadIdx.x == 0) {
-        target += gridDim.x;
-        ok = 1;
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const uint64_t t0 = now_ns();
-        while (ld_acquire(bar) < target) {
-            if (now_ns() - t0 > kWaitNs) {
-                atomicExch(err, 1);
-                ok = 0;
-                break;
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 __device__ __forceinline__ uint2 ld_rec(const uint2* p) {
     uint2 v;
     asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
@@ -328,14 +291,7 @@ __global__ void __launch_bounds__(kCT, 1) k_lanczos_cycle(CycleArgs<VT> a) {
         x = xn;
         __syncthreads();                             // w is written again by the next step
     }
-    // the last block out leaves the barrier as it found it
-    if (threadIdx.x == 0 && gridDim.x > 1) {
-        if (atomicAdd(a.bar + 1, 1u) == gridDim.x - 1) {
-            a.bar[0] = 0u;
-            a.bar[1] = 0u;
-            __threadfence();
-        }
-    }
+    barrier_exit(a.bar);
 }
 
 int cycle_sms() {

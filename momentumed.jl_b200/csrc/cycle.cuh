@@ -1,8 +1,57 @@
-// Cooperative kernel for the steps of a single-vector Lanczos cycle (cycle.cu).
+// Cooperative kernels for Lanczos steps: a single-vector cycle (cycle.cu), a step of the lockstep block
+// solver (blockstep.cu).
 #pragma once
 #include "vecops.cuh"
 
 namespace momed {
+
+#ifdef __CUDACC__
+constexpr uint64_t kWaitNs = 2000000000ull;   // a barrier gives up after two seconds
+__device__ __forceinline__ uint64_t now_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+// All blocks of the cooperative launch arrive; what they wrote before is visible after.  False (for
+// every thread of the block) when the wait ran out: the kernel then returns and the host reads err.
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& target, int* err) {
+    __shared__ int ok;
+    __syncthreads();
+    if (gridDim.x == 1) return true;
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        ok = 1;
+        __threadfence();
+        atomicAdd(bar, 1u);
+        const uint64_t t0 = now_ns();
+        while (ld_acquire(bar) < target) {
+            if (now_ns() - t0 > kWaitNs) {
+                atomicExch(err, 1);
+                ok = 0;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// the last block out leaves the barrier as it found it
+__device__ __forceinline__ void barrier_exit(unsigned* bar) {
+    if (threadIdx.x == 0 && gridDim.x > 1 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
+        bar[0] = 0u;
+        bar[1] = 0u;
+        __threadfence();
+    }
+}
+#endif
 
 enum CycleMap : int { CYCLE_NONE = 0, CYCLE_HITS = 1, CYCLE_CSR = 2 };
 

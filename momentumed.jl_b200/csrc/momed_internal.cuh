@@ -342,8 +342,7 @@ struct PairMap {
     DevBuf<uint4> tile;
     DevBuf<uint32_t> ent_row, row_ent;
     DevBuf<int4> work;
-    DevBuf<double2> psi64;     // workspace of a product, one value per entry
-    DevBuf<float2> psi32;
+    DevBuf<double2> psi;       // workspace of a product, one value per entry (FP32 products use half of it)
     PairView view() const;
     void release() {
         built = declined = false;
@@ -353,8 +352,7 @@ struct PairMap {
         ent_row.release();
         row_ent.release();
         work.release();
-        psi64.release();
-        psi32.release();
+        psi.release();
     }
 };
 

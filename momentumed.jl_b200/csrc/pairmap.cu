@@ -720,6 +720,7 @@ bool build_pair_map(momed_handle* h) {
     pm.n = n;
     pm.kmax = kmax;
     pm.entries = (int64_t)th[0];
+    pm.psi.resize(std::max<int64_t>(pm.entries, 1));   // here, so that the first product does not wait for it
     pm.hits = (int64_t)th[1];
     pm.bytes = nent * 4 + slots * 4 + tiles * 16;
     pm.built = true;
@@ -734,7 +735,6 @@ template <> struct PairSlot<double> {
     static DevBuf<double2>& d(PairPlan& p) { return p.d64; }
     static double& u(PairPlan& p) { return p.u64; }
     static bool& ok(PairPlan& p) { return p.ok64; }
-    static DevBuf<double2>& psi(PairMap& m) { return m.psi64; }
     static const double2* a(const OpView& o) { return o.t_amp; }
     static const double2* b(const OpView& o) { return o.t_ampb; }
 };
@@ -743,7 +743,6 @@ template <> struct PairSlot<float> {
     static DevBuf<float2>& d(PairPlan& p) { return p.d32; }
     static double& u(PairPlan& p) { return p.u32; }
     static bool& ok(PairPlan& p) { return p.ok32; }
-    static DevBuf<float2>& psi(PairMap& m) { return m.psi32; }
     static const float2* a(const OpView& o) { return o.t_amp32; }
     static const float2* b(const OpView& o) { return o.t_ampb32; }
 };
@@ -757,6 +756,7 @@ void ids_launch(const PairMap& pm, const PairPlan& pl, const typename Cx<R>::T* 
 template <typename R>
 void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* y, double u, cudaStream_t st) {
     using S = PairSlot<R>;
+    using C2 = typename Cx<R>::T;
     PairPlan& pl = h->pplan;
     PairMap& pm = h->hcache.pair;
     MOMED_REQUIRE(pm.built && pm.n == h->n, MOMED_ESTATE, "pair map: not built");
@@ -764,7 +764,7 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
     const OpView ov = h->op.view();
     auto& V = S::v(pl);
     auto& D = S::d(pl);
-    auto& psi = S::psi(pm);
+    C2* psi = reinterpret_cast<C2*>(pm.psi.p);
     if (!S::ok(pl) || (ov.t_ampb && S::u(pl) != u)) {         // formed again for another u or new amplitudes
         V.resize(std::max<int64_t>(pl.nv, 1));
         D.resize(64);
@@ -774,25 +774,24 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
         S::u(pl) = u;
         S::ok(pl) = true;
     }
-    psi.resize(std::max<int64_t>(pm.entries, 1));
     if (pm.nwork > 0) {
         // instantiated pair counts: every even one to 16 and the odd ones that meshes of 21 to 30
         // orbitals have (13, 15), then steps of 4; a class pads to the next
         switch (pl.pmax <= 4 ? 4 : pl.pmax <= 16 ? (pl.pmax == 13 || pl.pmax == 15 ? pl.pmax : (pl.pmax + 1) / 2 * 2)
                                                  : (pl.pmax + 3) / 4 * 4) {
-            case 4: ids_launch<R, 4>(pm, pl, V.p, x, psi.p, st); break;
-            case 6: ids_launch<R, 6>(pm, pl, V.p, x, psi.p, st); break;
-            case 8: ids_launch<R, 8>(pm, pl, V.p, x, psi.p, st); break;
-            case 10: ids_launch<R, 10>(pm, pl, V.p, x, psi.p, st); break;
-            case 12: ids_launch<R, 12>(pm, pl, V.p, x, psi.p, st); break;
-            case 13: ids_launch<R, 13>(pm, pl, V.p, x, psi.p, st); break;
-            case 14: ids_launch<R, 14>(pm, pl, V.p, x, psi.p, st); break;
-            case 15: ids_launch<R, 15>(pm, pl, V.p, x, psi.p, st); break;
-            case 16: ids_launch<R, 16>(pm, pl, V.p, x, psi.p, st); break;
-            case 20: ids_launch<R, 20>(pm, pl, V.p, x, psi.p, st); break;
-            case 24: ids_launch<R, 24>(pm, pl, V.p, x, psi.p, st); break;
-            case 28: ids_launch<R, 28>(pm, pl, V.p, x, psi.p, st); break;
-            default: ids_launch<R, 32>(pm, pl, V.p, x, psi.p, st); break;
+            case 4: ids_launch<R, 4>(pm, pl, V.p, x, psi, st); break;
+            case 6: ids_launch<R, 6>(pm, pl, V.p, x, psi, st); break;
+            case 8: ids_launch<R, 8>(pm, pl, V.p, x, psi, st); break;
+            case 10: ids_launch<R, 10>(pm, pl, V.p, x, psi, st); break;
+            case 12: ids_launch<R, 12>(pm, pl, V.p, x, psi, st); break;
+            case 13: ids_launch<R, 13>(pm, pl, V.p, x, psi, st); break;
+            case 14: ids_launch<R, 14>(pm, pl, V.p, x, psi, st); break;
+            case 15: ids_launch<R, 15>(pm, pl, V.p, x, psi, st); break;
+            case 16: ids_launch<R, 16>(pm, pl, V.p, x, psi, st); break;
+            case 20: ids_launch<R, 20>(pm, pl, V.p, x, psi, st); break;
+            case 24: ids_launch<R, 24>(pm, pl, V.p, x, psi, st); break;
+            case 28: ids_launch<R, 28>(pm, pl, V.p, x, psi, st); break;
+            default: ids_launch<R, 32>(pm, pl, V.p, x, psi, st); break;
         }
         MOMED_CUDA_TRY(cudaGetLastError());
         note_launches(1);
@@ -802,7 +801,7 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
     int G = 1;
     while (G < 8 && rw * G < want) G *= 2;
     const int per = kPT / 32 / G;
-    k_pair_rows<R><<<(unsigned)((rw + per - 1) / per), kPT, 0, st>>>(pm.view(), h->basis.p, D.p, psi.p, x, y, G);
+    k_pair_rows<R><<<(unsigned)((rw + per - 1) / per), kPT, 0, st>>>(pm.view(), h->basis.p, D.p, psi, x, y, G);
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
 }

@@ -23,6 +23,7 @@
 #include <thread>
 #include <type_traits>
 
+#include "blockcombine.cuh"
 #include "blockstep.cuh"
 
 namespace momed {
@@ -264,65 +265,6 @@ __global__ void k_brandom(VT* v, int64_t total, uint64_t seed) {
     }
 }
 
-// out[i][n][r] = sum_a U[i][a][r] V[a][n][r]  (U: [nout][m][NB] real, r fastest so a warp's
-// coefficient loads are coalesced), optionally out[nout] = V[copy_col].  Each thread owns RPT rows
-// of one right-hand side and accumulates OC outputs at a time in registers of type ACC, streaming
-// V straight from HBM (the unrolled a-loop keeps several loads in flight).  out must not overlap V.
-template <typename VIN, typename VOUT, typename ACC, int NB, int RPT, int OC>
-__global__ void __launch_bounds__(kT)
-k_bcombine(const VIN* __restrict__ V, int64_t N, int m, const double* __restrict__ U, int nout,
-           VOUT* __restrict__ out, int copy_col) {
-    constexpr int TPR = kT / NB;        // row slots per block pass
-    const int r = threadIdx.x % NB, slot = threadIdx.x / NB;
-    const int64_t stride = N * NB;
-    for (int64_t t0 = (int64_t)blockIdx.x * TPR * RPT; t0 < N; t0 += (int64_t)gridDim.x * TPR * RPT) {
-        int64_t off[RPT];
-        bool ok[RPT];
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-            const int64_t row = t0 + slot + (int64_t)j * TPR;
-            ok[j] = row < N;
-            off[j] = (ok[j] ? row : 0) * NB + r;
-        }
-        for (int c0 = 0; c0 < nout; c0 += OC) {
-            ACC ax[RPT][OC], ay[RPT][OC];
-#pragma unroll
-            for (int j = 0; j < RPT; ++j)
-#pragma unroll
-                for (int k = 0; k < OC; ++k) { ax[j][k] = 0; ay[j][k] = 0; }
-#pragma unroll 2
-            for (int a = 0; a < m; ++a) {
-                ACC u[OC];
-#pragma unroll
-                for (int k = 0; k < OC; ++k)
-                    u[k] = (c0 + k < nout) ? (ACC)__ldg(U + ((int64_t)(c0 + k) * m + a) * NB + r) : (ACC)0;
-#pragma unroll
-                for (int j = 0; j < RPT; ++j) {
-                    const VIN v = V[(int64_t)a * stride + off[j]];
-#pragma unroll
-                    for (int k = 0; k < OC; ++k) {
-                        ax[j][k] += u[k] * (ACC)v.x;
-                        ay[j][k] += u[k] * (ACC)v.y;
-                    }
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < RPT; ++j) {
-                if (!ok[j]) continue;
-#pragma unroll
-                for (int k = 0; k < OC; ++k)
-                    if (c0 + k < nout)
-                        out[(int64_t)(c0 + k) * stride + off[j]] = from_d2<VOUT>(make_double2((double)ax[j][k], (double)ay[j][k]));
-            }
-        }
-        if (copy_col >= 0) {
-#pragma unroll
-            for (int j = 0; j < RPT; ++j)
-                if (ok[j]) out[(int64_t)nout * stride + off[j]] = from_d2<VOUT>(to_d2(V[(int64_t)copy_col * stride + off[j]]));
-        }
-    }
-}
-
 template <int NB>
 __global__ void k_binv(const double2* c, double* scal) {
     int r = threadIdx.x;
@@ -447,6 +389,8 @@ struct BlockLanczos {
     // replay them, stay for per-launch timing and MOMED_COOP=0.
     bool coopb = false;
     BlockStepBufs<VT> bs;
+    // set on the device by a cooperative step whose grid barrier gave up; none with the separate kernels
+    const int* err_flag() const { return coop ? cy.a.err : coopb ? bs.a.err : nullptr; }
 
     ~BlockLanczos() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
@@ -516,7 +460,6 @@ struct BlockLanczos {
         scal.resize(NB);
         alpha.resize((size_t)NB * m);
         beta.resize((size_t)NB * m);
-        Ud.resize((size_t)NB * m * m);
         flag.resize(NB);
         any.resize(1);
         if (want_coop && cy.prepare(N, false, alpha.p, beta.p, dgks, st)) {
@@ -611,18 +554,7 @@ struct BlockLanczos {
     }
     template <typename VOUT>
     void combine(const std::vector<double>& Uh, int nout, VOUT* out, int copy_col, int mm) {
-        MOMED_CUDA_TRY(cudaMemcpyAsync(Ud.p, Uh.data(), Uh.size() * 8, cudaMemcpyHostToDevice, st));
-        // FP32 accumulation when FP32 vectors are recombined into FP32 vectors; FP64 otherwise
-        constexpr bool f32 = std::is_same<VT, float2>::value && std::is_same<VOUT, float2>::value;
-        using ACC = typename std::conditional<f32, float, double>::type;
-        constexpr int RPT = f32 ? 4 : 2;
-        constexpr int TR = (kT / NB) * RPT;
-        // (one pass of 16 outputs and 2 rows per thread for 9..16 outputs was slower: 1.61 against
-        // 1.21 ms for the headline restart's 12)
-        auto k = k_bcombine<VT, VOUT, ACC, NB, RPT, 8>;
-        int g = (int)std::max<int64_t>(1, std::min<int64_t>((N + TR - 1) / TR, (int64_t)sms() * 8));
-        k<<<g, kT, 0, st>>>(V.p, N, mm, Ud.p, nout, out, copy_col);
-        MOMED_CUDA_TRY(cudaGetLastError());
+        block_combine<VT, VOUT>(V.p, N, NB, mm, Uh, nout, out, copy_col, Ud, st);
         MOMED_CUDA_TRY(cudaStreamSynchronize(st));
         ++launches;
     }
@@ -679,8 +611,7 @@ struct BlockLanczos {
             MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
             MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
             int err = 0;
-            if (coop || coopb)
-                MOMED_CUDA_TRY(cudaMemcpyAsync(&err, coop ? cy.a.err : bs.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            if (const int* e = err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));
             MOMED_CUDA_TRY(cudaStreamSynchronize(st));
             CycleBufs<VT>::check(err);
             // per right-hand side projected eigenproblems, in parallel on the host
@@ -766,26 +697,6 @@ struct BlockLanczos {
     }
 };
 
-// out[i][n][r] = sum_a Y[r][i][a] X[a][n][r]   (Y: [NB][k][k] complex, out != X)
-template <int NB>
-__global__ void k_bcombine_c(const double2* __restrict__ X, int64_t N, int k, const double2* __restrict__ Y,
-                             double2* __restrict__ out) {
-    const int64_t total = N * NB;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(e % NB);
-        for (int i = 0; i < k; ++i) {
-            double sx = 0.0, sy = 0.0;
-            for (int a = 0; a < k; ++a) {
-                double2 y = Y[((int64_t)r * k + i) * k + a];
-                double2 x = X[(int64_t)a * total + e];
-                sx += y.x * x.x - y.y * x.y;
-                sy += y.x * x.y + y.y * x.x;
-            }
-            out[(int64_t)i * total + e] = make_double2(sx, sy);
-        }
-    }
-}
-
 // out[n][r] = sum_{i < k} X[i][n][r]  (warm-start block from refined Ritz vectors)
 template <int NB>
 __global__ void k_bsum(const double2* __restrict__ X, int64_t N, int k, double2* __restrict__ out) {
@@ -851,93 +762,6 @@ __global__ void k_bto(const double2* __restrict__ X, int64_t total, VT* __restri
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x)
         out[e] = from_d2<VT>(X[e]);
 }
-
-// out[i][n][r] = sum_{a<kx} Y[i][a][r] X[a][n][r] + sum_{b<kz} Y[i][kx+b][r] Z[b][n][r]
-//               + sum_{j<p} Y[i][kx+kz+j][r] Q[j][n][r]
-// (Y complex, [(i * (kx + kz + p) + a) * NB + r]; FP64 sources X and Z, FP32 source Q; FP64 out).
-// A thread owns RPT rows of one right-hand side, so each coefficient load serves RPT rows.
-template <int NB>
-__global__ void __launch_bounds__(kT, 2)
-k_bcombine_xq(const double2* __restrict__ X, int kx, const double2* __restrict__ Z, int kz,
-              const float2* __restrict__ Q, int p, int64_t N, const double2* __restrict__ Y, int nout,
-              double2* __restrict__ out) {
-    constexpr int OC = 8, RPT = 2;
-    constexpr int TPR = kT / NB;        // row slots per block pass
-    const int d = kx + kz + p;
-    const int64_t stride = N * NB;
-    const int r = threadIdx.x % NB, slot = threadIdx.x / NB;
-    for (int64_t t0 = (int64_t)blockIdx.x * TPR * RPT; t0 < N; t0 += (int64_t)gridDim.x * TPR * RPT) {
-        int64_t off[RPT];
-        bool ok[RPT];
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-            const int64_t row = t0 + slot + (int64_t)j * TPR;
-            ok[j] = row < N;
-            off[j] = (ok[j] ? row : 0) * NB + r;
-        }
-        for (int c0 = 0; c0 < nout; c0 += OC) {
-            double ax[RPT][OC], ay[RPT][OC];
-#pragma unroll
-            for (int j = 0; j < RPT; ++j)
-#pragma unroll
-                for (int k = 0; k < OC; ++k) { ax[j][k] = 0.0; ay[j][k] = 0.0; }
-            {
-                // the FP32 extension Q in FP32 arithmetic (its values carry FP32 rounding already;
-                // the products add an error of the same order), summed into the FP64 sums after
-                float fx[RPT][OC], fy[RPT][OC];
-#pragma unroll
-                for (int j = 0; j < RPT; ++j)
-#pragma unroll
-                    for (int k = 0; k < OC; ++k) { fx[j][k] = 0.f; fy[j][k] = 0.f; }
-                for (int a = kx + kz; a < d; ++a) {
-                    float2 y[OC];
-#pragma unroll
-                    for (int k = 0; k < OC; ++k) {
-                        const double2 yd = (c0 + k < nout) ? __ldg(Y + ((int64_t)(c0 + k) * d + a) * NB + r)
-                                                           : make_double2(0.0, 0.0);
-                        y[k] = make_float2((float)yd.x, (float)yd.y);
-                    }
-#pragma unroll
-                    for (int j = 0; j < RPT; ++j) {
-                        const float2 v = Q[(int64_t)(a - kx - kz) * stride + off[j]];
-#pragma unroll
-                        for (int k = 0; k < OC; ++k) {
-                            fx[j][k] += y[k].x * v.x - y[k].y * v.y;
-                            fy[j][k] += y[k].x * v.y + y[k].y * v.x;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < RPT; ++j)
-#pragma unroll
-                    for (int k = 0; k < OC; ++k) { ax[j][k] = (double)fx[j][k]; ay[j][k] = (double)fy[j][k]; }
-            }
-            for (int a = 0; a < kx + kz; ++a) {            // the FP64 anchors X (and Z)
-                double2 y[OC];
-#pragma unroll
-                for (int k = 0; k < OC; ++k)
-                    y[k] = (c0 + k < nout) ? __ldg(Y + ((int64_t)(c0 + k) * d + a) * NB + r) : make_double2(0.0, 0.0);
-#pragma unroll
-                for (int j = 0; j < RPT; ++j) {
-                    const double2 v = a < kx ? X[(int64_t)a * stride + off[j]] : Z[(int64_t)(a - kx) * stride + off[j]];
-#pragma unroll
-                    for (int k = 0; k < OC; ++k) {
-                        ax[j][k] += y[k].x * v.x - y[k].y * v.y;
-                        ay[j][k] += y[k].x * v.y + y[k].y * v.x;
-                    }
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < RPT; ++j) {
-                if (!ok[j]) continue;
-#pragma unroll
-                for (int k = 0; k < OC; ++k)
-                    if (c0 + k < nout) out[(int64_t)(c0 + k) * stride + off[j]] = make_double2(ax[j][k], ay[j][k]);
-            }
-        }
-    }
-}
-
 
 // Inner products of ncols columns of V with up to kGramRhs right-hand-side blocks at once:
 // partial[b][j][i][r] = block's sum over rows of conj(V_i[n][r]) R_j[n][r].  Grid: x = row blocks,
@@ -1125,7 +949,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
         }
         std::vector<double2> Yh((size_t)NB * k1 * k1, make_double2(0.0, 0.0));
         for (int q = 0; q < NB; ++q)
-            for (int i = 0; i < k1; ++i) Yh[((size_t)q * k1 + i) * k1 + i] = make_double2(1.0, 0.0);
+            for (int i = 0; i < k1; ++i) Yh[((size_t)i * k1 + i) * NB + q] = make_double2(1.0, 0.0);
         host_parallel(nu, [&](int q) {
             if (broken[q]) return;
             std::vector<double> t;
@@ -1135,15 +959,13 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
             for (int i = 0; i < k1; ++i)
                 for (int a = 0; a < k1; ++a) {
                     auto y = Y[(size_t)i * k1 + a];
-                    Yh[((size_t)q * k1 + i) * k1 + a] = make_double2(y.real(), y.imag());
+                    Yh[((size_t)i * k1 + a) * NB + q] = make_double2(y.real(), y.imag());
                 }
         });
         DevBuf<double2> Yd;
-        Yd.resize(Yh.size());
-        MOMED_CUDA_TRY(cudaMemcpyAsync(Yd.p, Yh.data(), Yh.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
-        k_bcombine_c<NB><<<eg, 256, 0, st>>>(Xb.p, N, k1, Yd.p, Sb.p);
+        block_combine_c(Xb.p, k1, nullptr, 0, nullptr, 0, N, NB, Yh, k1, Sb.p, Yd, st);
         Xb.swap(Sb);
-        k_bcombine_c<NB><<<eg, 256, 0, st>>>(Wb.p, N, k1, Yd.p, Sb.p);
+        block_combine_c(Wb.p, k1, nullptr, 0, nullptr, 0, N, NB, Yh, k1, Sb.p, Yd, st);
         Wb.swap(Sb);
         note_launches(2);
         MOMED_CUDA_TRY(cudaGetLastError());
@@ -1225,8 +1047,6 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
             thd.resize((size_t)NB * k1);
             wtd.resize((size_t)NB * k1);
             DevBuf<double2> Yd, Y2d, W2;
-            Yd.resize((size_t)k1 * d * NB);
-            Y2d.resize((size_t)k1 * d2 * NB);
             W2.resize((size_t)k1 * stride);
             // Gram partials [row block][kGramRhs][columns][NB] and the summed blocks [2 k1][columns][NB]
             DevBuf<double2> gpart, gx, gq;
@@ -1334,7 +1154,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                     gram(LR.col(k1), true, p, g0, nr, gq.p + (size_t)g0 * p * NB);       // q_j^H rhs
                 }
                 int err = 0;
-                if (LR.coop) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, LR.cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+                if (const int* e = LR.err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));
                 std::vector<double2> hx((size_t)gx_n), hq((size_t)gq_n);
                 MOMED_CUDA_TRY(cudaMemcpyAsync(hx.data(), gx.p, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
                 MOMED_CUDA_TRY(cudaMemcpyAsync(hq.data(), gq.p, hq.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
@@ -1419,13 +1239,9 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                         Y2h[((size_t)i * d2 + i) * NB + q] = make_double2(1.0, 0.0);
                     }
                 }
-                MOMED_CUDA_TRY(cudaMemcpyAsync(Yd.p, Yh.data(), Yh.size() * sizeof(double2), cudaMemcpyHostToDevice, st));
-                MOMED_CUDA_TRY(cudaMemcpyAsync(Y2d.p, Y2h.data(), Y2h.size() * sizeof(double2), cudaMemcpyHostToDevice,
-                                               st));
                 // X' = [X Q] Y and W' from the Lanczos relation (both read the old X and W)
-                const int xg = std::max(1, std::min<int>((int)((N + 2 * (kT / NB) - 1) / (2 * (kT / NB))), sms() * 8));
-                k_bcombine_xq<NB><<<xg, kT, 0, st>>>(Xb.p, k1, nullptr, 0, LR.col(k1), p, N, Yd.p, k1, Sb.p);
-                k_bcombine_xq<NB><<<xg, kT, 0, st>>>(Wb.p, k1, Xb.p, k1, LR.col(k1), p + 1, N, Y2d.p, k1, W2.p);
+                block_combine_c(Xb.p, k1, nullptr, 0, LR.col(k1), p, N, NB, Yh, k1, Sb.p, Yd, st);
+                block_combine_c(Wb.p, k1, Xb.p, k1, LR.col(k1), p + 1, N, NB, Y2h, k1, W2.p, Y2d, st);
                 note_launches(2);
                 MOMED_CUDA_TRY(cudaGetLastError());
                 Xb.swap(Sb);

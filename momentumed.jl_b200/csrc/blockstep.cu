@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "blockstep.cuh"
+#include "packets.cuh"
 
 namespace momed {
 
@@ -46,16 +47,6 @@ __device__ __forceinline__ double wred(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kAll, v, o);
     return v;
 }
-
-// Asynchronous copies of a thread's own packets to its own places of a ring in shared memory: no other
-// thread reads them, so a thread waits for its own copies only.
-template <typename PT> __device__ __forceinline__ void copy_packet(PT* dst, const PT* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    if constexpr (sizeof(PT) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // part[(c NB + r)][block] for c < ncols (and |w_r|^2 as c = ncols when norm).  The columns are dealt to
 // par groups of ch warps; the warps of a group take turns in rows.

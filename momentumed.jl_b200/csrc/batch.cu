@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "blockcombine.cuh"
+#include "blockgram.cuh"
 #include "blockstep.cuh"
 
 namespace momed {
@@ -763,107 +764,6 @@ __global__ void k_bto(const double2* __restrict__ X, int64_t total, VT* __restri
         out[e] = from_d2<VT>(X[e]);
 }
 
-// Inner products of ncols columns of V with up to kGramRhs right-hand-side blocks at once:
-// partial[b][j][i][r] = block's sum over rows of conj(V_i[n][r]) R_j[n][r].  Grid: x = row blocks,
-// y = groups of 8 columns (warp per column, as in k_bproj); every column packet read from HBM
-// serves all right-hand sides, which the block's warps share through L1.
-constexpr int kGramRhs = 4;
-struct GramRhs {
-    const double2* p[kGramRhs];
-};
-template <typename VT, int NB>
-__global__ void __launch_bounds__(kT, 4)
-k_bgram(const VT* __restrict__ V, int64_t N, int ncols, GramRhs R, int nr, double2* __restrict__ partial) {
-    using P = Pack<VT, NB>;
-    constexpr int E = P::E;
-    constexpr int PR = NB / E;
-    constexpr int RS = 32 / PR;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int rp = lane % PR, rs = lane / PR;
-    const int i = blockIdx.y * 8 + wid;
-    if (i >= ncols) return;                     // warp-uniform
-    double ax[kGramRhs][E], ay[kGramRhs][E];
-#pragma unroll
-    for (int j = 0; j < kGramRhs; ++j)
-#pragma unroll
-        for (int q = 0; q < E; ++q) { ax[j][q] = 0.0; ay[j][q] = 0.0; }
-    const int64_t per = (N + gridDim.x - 1) / gridDim.x;
-    const int64_t r0 = (int64_t)blockIdx.x * per, r1 = min(N, r0 + per);
-    const typename P::T* col = reinterpret_cast<const typename P::T*>(V + (int64_t)i * N * NB);
-#pragma unroll 2
-    for (int64_t t = r0 + rs; t < r1; t += RS) {
-        double2 v[E];
-        P::get(col[t * PR + rp], v);
-#pragma unroll
-        for (int j = 0; j < kGramRhs; ++j) {
-            if (j < nr) {
-#pragma unroll
-                for (int q = 0; q < E; ++q) {
-                    const double2 w = __ldg(R.p[j] + t * NB + rp * E + q);
-                    ax[j][q] += v[q].x * w.x + v[q].y * w.y;
-                    ay[j][q] += v[q].x * w.y - v[q].y * w.x;
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < kGramRhs; ++j) {
-#pragma unroll
-        for (int q = 0; q < E; ++q) {
-            double sx = ax[j][q], sy = ay[j][q];
-#pragma unroll
-            for (int o = PR; o < 32; o <<= 1) {
-                sx += __shfl_xor_sync(0xffffffffu, sx, o);
-                sy += __shfl_xor_sync(0xffffffffu, sy, o);
-            }
-            if (j < nr && rs == 0)
-                partial[(((int64_t)blockIdx.x * kGramRhs + j) * ncols + i) * NB + rp * E + q] = make_double2(sx, sy);
-        }
-    }
-}
-
-// Row blocks of k_bgram: one wave of the CTAs that are resident at once over the ncols / 8
-// column groups (measured: a grid of 0.67 or 3 waves left the SMs a third idle or ran a partial
-// last wave), at least one row tile each, at most cap.
-constexpr int kGramBlocksPerSm = 8;
-template <int NB>
-int gram_rowblocks_t(int64_t N, int ncols, bool fp32, int cap) {
-    static std::atomic<int> per_sm[2];   // zero before first use (static storage)
-    int ps = per_sm[fp32 ? 1 : 0].load(std::memory_order_relaxed);
-    if (ps == 0) {
-        if (fp32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_bgram<float2, NB>, kT, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_bgram<double2, NB>, kT, 0);
-        if (ps <= 0) ps = 1;
-        per_sm[fp32 ? 1 : 0].store(ps, std::memory_order_relaxed);
-    }
-    int sm = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
-    if (sm <= 0) sm = 148;
-    const int groups = std::max(1, (ncols + 7) / 8);
-    int rb = std::max(1, ps * sm / groups);
-    rb = (int)std::min<int64_t>(rb, (N + rows_tile<NB>() - 1) / rows_tile<NB>());
-    return std::max(1, std::min(rb, cap));
-}
-
-// out[e] = sum over blocks b < grid of partial[b * bstride + e] for e < count, one warp per
-// element (fixed order)
-__global__ void k_bsum_blocks(const double2* __restrict__ partial, int grid, int64_t bstride, int64_t count,
-                              double2* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t e = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (e >= count) return;
-    double sx = 0.0, sy = 0.0;
-    for (int b = lane; b < grid; b += 32) {
-        const double2 v = partial[(int64_t)b * bstride + e];
-        sx += v.x;
-        sy += v.y;
-    }
-    sx = wsum(sx);
-    sy = wsum(sy);
-    if (lane == 0) out[e] = make_double2(sx, sy);
-}
-
 template <int NB>
 int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32_t nu, double* vals, double* resid,
               double* vecs, momed_info* info) {
@@ -927,26 +827,29 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
     const int eg = std::max(1, std::min<int>((int)((stride + 255) / 256), sms() * 8));
     if (mixed) {
         // Gram matrices G_r = X_r^H W_r and S_r = X_r^H X_r, all r at once
-        const int grid = std::max(1, std::min<int>((int)((N + rows_tile<NB>() - 1) / rows_tile<NB>()), sms() * 2));
         DevBuf<double2> part, red;
-        part.resize((size_t)grid * (kMaxCols + 1) * NB);
-        red.resize((size_t)(kMaxCols + 1) * NB);
+        part.resize(block_gram_part(NB, k1));
+        const size_t per = (size_t)k1 * NB;                       // one right-hand side against X
+        red.resize(2 * k1 * per);
         std::vector<std::vector<std::complex<double>>> G(NB, std::vector<std::complex<double>>((size_t)k1 * k1)),
             S(NB, std::vector<std::complex<double>>((size_t)k1 * k1));
-        std::vector<double2> hr((size_t)(k1 + 1) * NB);
-        for (int pass = 0; pass < 2; ++pass) {
-            for (int i = 0; i < k1; ++i) {
-                const double2* rhs = (pass == 0 ? Wb.p : Xb.p) + (size_t)i * stride;
-                k_bproj<double2, double2, NB><<<bproj_grid(grid, k1), kT, 0, st>>>(Xb.p, N, k1, rhs, part.p, nullptr);
-                k_breduce<NB><<<breduce_grid(k1 + 1, NB), 256, 0, st>>>(part.p, grid, k1 + 1, red.p, nullptr);
-                note_launches(2);
-                MOMED_CUDA_TRY(cudaMemcpyAsync(hr.data(), red.p, hr.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
-                MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-                for (int q = 0; q < nu; ++q)
-                    for (int a = 0; a < k1; ++a)
-                        (pass == 0 ? G : S)[q][(size_t)i * k1 + a] = std::complex<double>(hr[a * NB + q].x, hr[a * NB + q].y);
-            }
+        for (int j0 = 0; j0 < 2 * k1; j0 += kGramRhs) {           // W_0 .. W_{k1-1}, X_0 .. X_{k1-1}
+            const int nr = std::min(kGramRhs, 2 * k1 - j0);
+            const double2* rhs[kGramRhs];
+            for (int j = 0; j < nr; ++j)
+                rhs[j] = j0 + j < k1 ? Wb.p + (size_t)(j0 + j) * stride : Xb.p + (size_t)(j0 + j - k1) * stride;
+            block_gram(Xb.p, N, NB, k1, rhs, nr, part.p, red.p + j0 * per, st);
+            note_launches(2);
         }
+        std::vector<double2> hr(2 * k1 * per);
+        MOMED_CUDA_TRY(cudaMemcpyAsync(hr.data(), red.p, hr.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
+        MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+        for (int j = 0; j < 2 * k1; ++j)
+            for (int q = 0; q < nu; ++q)
+                for (int a = 0; a < k1; ++a) {
+                    const double2 v = hr[j * per + (size_t)a * NB + q];
+                    (j < k1 ? G : S)[q][(size_t)(j % k1) * k1 + a] = std::complex<double>(v.x, v.y);
+                }
         std::vector<double2> Yh((size_t)NB * k1 * k1, make_double2(0.0, 0.0));
         for (int q = 0; q < NB; ++q)
             for (int i = 0; i < k1; ++i) Yh[((size_t)i * k1 + i) * NB + q] = make_double2(1.0, 0.0);
@@ -1048,12 +951,9 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
             wtd.resize((size_t)NB * k1);
             DevBuf<double2> Yd, Y2d, W2;
             W2.resize((size_t)k1 * stride);
-            // Gram partials [row block][kGramRhs][columns][NB] and the summed blocks [2 k1][columns][NB]
+            // Gram partials of the blocks, and the summed products [2 k1][columns][NB]
             DevBuf<double2> gpart, gx, gq;
-            // Gram row blocks: one wave of resident CTAs over all column groups (occupancy of
-            // k_bgram), up to kGramBlocksPerSm per SM; the partial buffer holds that many
-            const int gram_cap = kGramBlocksPerSm * sms();
-            gpart.resize((size_t)gram_cap * kGramRhs * std::max(k1, m - k1) * NB);
+            gpart.resize(std::max(block_gram_part(NB, k1), block_gram_part(NB, m - k1)));
             const size_t gx_n = (size_t)2 * k1 * k1 * NB, gq_n = (size_t)2 * k1 * (m - k1) * NB;
             gx.resize(gx_n);
             gq.resize(gq_n);
@@ -1131,27 +1031,14 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                 // FP64 Gram blocks: b_a^H H b_i and b_a^H b_i for the anchors i against [X, Q]; the
                 // 2 k1 right-hand sides (W_i, then X_i) go kGramRhs at a time
                 const int nrhs = 2 * k1;
-                auto gram = [&](const void* cols, bool fp32, int ncols, int g0, int nr, double2* out) {
-                    const int rb = gram_rowblocks_t<NB>(N, ncols, fp32, gram_cap);
-                    GramRhs R{};
-                    for (int j = 0; j < nr; ++j)
-                        R.p[j] = (g0 + j < k1 ? Wb.p + (size_t)(g0 + j) * stride : Xb.p + (size_t)(g0 + j - k1) * stride);
-                    for (int j = nr; j < kGramRhs; ++j) R.p[j] = R.p[0];
-                    if (fp32)
-                        k_bgram<float2, NB><<<bproj_grid(rb, ncols), kT, 0, st>>>(
-                            reinterpret_cast<const float2*>(cols), N, ncols, R, nr, gpart.p);
-                    else
-                        k_bgram<double2, NB><<<bproj_grid(rb, ncols), kT, 0, st>>>(
-                            reinterpret_cast<const double2*>(cols), N, ncols, R, nr, gpart.p);
-                    // the nr valid slabs lead each block's [kGramRhs][ncols][NB] partials
-                    const int64_t bstride = (int64_t)kGramRhs * ncols * NB, count = (int64_t)nr * ncols * NB;
-                    k_bsum_blocks<<<(unsigned)((count + 7) / 8), 256, 0, st>>>(gpart.p, rb, bstride, count, out);
-                    note_launches(2);
-                };
                 for (int g0 = 0; g0 < nrhs; g0 += kGramRhs) {
                     const int nr = std::min(kGramRhs, nrhs - g0);
-                    gram(Xb.p, false, k1, g0, nr, gx.p + (size_t)g0 * k1 * NB);          // x_a^H rhs
-                    gram(LR.col(k1), true, p, g0, nr, gq.p + (size_t)g0 * p * NB);       // q_j^H rhs
+                    const double2* rhs[kGramRhs];
+                    for (int j = 0; j < nr; ++j)
+                        rhs[j] = g0 + j < k1 ? Wb.p + (size_t)(g0 + j) * stride : Xb.p + (size_t)(g0 + j - k1) * stride;
+                    block_gram(Xb.p, N, NB, k1, rhs, nr, gpart.p, gx.p + (size_t)g0 * k1 * NB, st);     // x_a^H rhs
+                    block_gram(LR.col(k1), N, NB, p, rhs, nr, gpart.p, gq.p + (size_t)g0 * p * NB, st); // q_j^H rhs
+                    note_launches(4);
                 }
                 int err = 0;
                 if (const int* e = LR.err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -1,5 +1,6 @@
-"""The recombinations of the lockstep block solver (csrc/blockcombine.cu) against LAPACK at the edges of
-their output tiles: 1 to 20 wanted pairs (kept combinations and Ritz vectors of one tile, a full one,
+"""The recombinations of the lockstep block solver (csrc/blockcombine.cu) and its Gram blocks
+(csrc/blockgram.cu: 5 to 24 FP64 columns, 11 to 46 FP32 ones, so one pass of 32 columns and two) against
+LAPACK at the edges of their tiles: 1 to 20 wanted pairs (kept combinations and Ritz vectors of one tile, a full one,
 two and three), bases that are no multiple of a run of sources, an odd and an even number of rows, and
 block widths with one and two values per packet, in both precisions.
 

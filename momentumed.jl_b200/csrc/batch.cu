@@ -582,13 +582,15 @@ struct BlockLanczos {
     Out run(int nev, int nu, double tol, double rel_floor, int maxiter, uint64_t seed, int nwant, double2* vectors,
             const VT* start = nullptr, double eig_target = 0.0) {
         Out out;
-        // The classical 1/2 (|w'| < 0.71 |w|) flags nearly every Lanczos step, because w = H v
-        // carries alpha and beta along the two newest columns, and one flagged right-hand side
-        // makes the whole block repeat the pass.  Measured on B200: with FP64 bases, or few
-        // wanted pairs (nev <= m/5), 0.1 runs the same maps and gives the same eigenvalues as
-        // 1/2 (3x9, 32 U0, nev 4: 16% faster; 0.01 the same); an FP32 basis with nev 12 in m 36
-        // needed 1.65x the maps at 0.1, so FP32 with more wanted pairs keeps 1/2.
-        dgks = (std::is_same<VT, float2>::value && 5 * nev > m) ? 0.5 : 0.1;
+        // The classical 1/2 (|w'| < 0.71 |w|) flags about half of all Lanczos steps, because w = H v
+        // carries beta along the two neighbouring columns (|w'|^2 / |w|^2 of a step is 0.45 to 0.55),
+        // and one flagged right-hand side makes the whole block repeat the pass.  Measured on B200:
+        // with FP64 bases, or few wanted pairs (nev <= m/5), 0.1 runs the same maps and gives the same
+        // eigenvalues as 1/2 (3x9, 32 U0, nev 4: 16% faster; 0.01 the same).  FP32 bases with more
+        // wanted pairs take 0.2: over 3x8, 3x9 and 4x6 sectors, 1 and 8 right-hand sides, nev 7 to 20
+        // in m 24 to 64 and three seeds the maps are those of 1/2 (within a restart cycle either way)
+        // and the time 2 to 25% less: 3x9, nev 7 in m 30 41.3 -> 37.3 ms alone, 191 -> 162 ms for 8.
+        dgks = (std::is_same<VT, float2>::value && 5 * nev > m) ? 0.2 : 0.1;
         // graphs captured by an earlier run of this object carry that run's dgks: capture anew
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
         graphs.clear();
@@ -945,7 +947,7 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
             const int p = m - k1, d = k1 + p;
             const int d2 = 2 * k1 + p + 1;     // sources of W': W, X, Q and the next Lanczos vector
             BlockLanczos<float2, NB> LR(h, m, uv);
-            LR.dgks = 5 * nev > m ? 0.5 : 0.1;   // the rule of BlockLanczos::run for an FP32 basis
+            LR.dgks = 5 * nev > m ? 0.2 : 0.1;   // the rule of BlockLanczos::run for an FP32 basis
             DevBuf<double> thd, wtd;
             thd.resize((size_t)NB * k1);
             wtd.resize((size_t)NB * k1);

@@ -533,7 +533,6 @@ def run_plain_workload(args, rank, world, local):
         solve(order[i], _lib.PREC_FP64)
     torch.cuda.synchronize()
     launches0 = _lib.kernel_launches()
-    h.profile(True)
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(K + 1)]
     infos, vals64 = [], []
     barrier(world)
@@ -548,6 +547,14 @@ def run_plain_workload(args, rank, world, local):
         torch.cuda.synchronize()
     barrier(world)
     step_ms = [ev[i].elapsed_time(ev[i + 1]) for i in range(K)]
+    launches = _lib.kernel_launches() - launches0
+    # device time of the maps: the first (up to 3) timed sectors again with per-launch events, which
+    # need separate launches (the timed solves run their steps as cooperative kernels, some with the
+    # map inside)
+    h.profile(True)
+    for i in range(min(K, 3)):
+        solve(order[W + i], _lib.PREC_FP64)
+    torch.cuda.synchronize()
     n_mv, ms_mv = h.profile_read(_lib.KERNEL_SPMV_C128 if sparse else _lib.KERNEL_MATVEC_C128)
     n_bmv, ms_bmv = h.profile_read(_lib.KERNEL_BLOCK_MATVEC_C128)
     n_hmv, ms_hmv = h.profile_read(_lib.KERNEL_HC_MATVEC_C128)
@@ -561,7 +568,8 @@ def run_plain_workload(args, rank, world, local):
     bsz = block_size(nev, len(sectors[order[W]][1])) if not sparse else 0
     if bsz and n_bmv > 0:
         n_mv, ms_mv = n_bmv, ms_bmv
-    launches = _lib.kernel_launches() - launches0
+    else:
+        bsz = 0                                        # over the pair tables: the single-vector solver
     elapsed = all_max(sum(step_ms) / 1e3, world)
     value = all_sum(K, world) / elapsed
     nb, nnz_mean, build_ms, hc_info = [], [], [], []
@@ -572,7 +580,9 @@ def run_plain_workload(args, rank, world, local):
         if use_hc:
             hc = h.build_hit_cache()
             hc_info.append(hc)
-            nb.append(hc_bytes(len(sectors[sidx][1]), hc["hits"], len(pair[0]), max(bsz, 1), 16))
+            pairs = 0 if bsz else pair_table_bytes(hc, len(sectors[sidx][1]))
+            nb.append(pair_bytes(pairs, sum(w["N_each"]), len(sectors[sidx][1]), 16) if pairs > 0 else
+                      hc_bytes(len(sectors[sidx][1]), hc["hits"], len(pair[0]), max(bsz, 1), 16))
             nnz_mean.append(st["nnz"])
         elif sparse:
             torch.cuda.synchronize()
@@ -653,7 +663,8 @@ def run_plain_workload(args, rank, world, local):
                       else f"block map c128 x{bsz} (k_block_matvec_v<double, {bsz}>, block Lanczos)")
             extra = {"block_lanczos": {"block": bsz, "maps_per_launch": bsz}}
         else:
-            kernel = "map c128 over the hit cache (k_matvec_hc<double>)" if use_hc else "map c128 (k_matvec<double>)"
+            kernel = ("map c128 over the pair tables (k_pair_ids, k_pair_rows)" if use_hc and pairs > 0 else
+                      "map c128 over the hit cache (k_matvec_hc<double>)" if use_hc else "map c128 (k_matvec<double>)")
             extra = {}
         if use_hc:
             extra["hit_cache"] = {"hits_per_sector": float(np.mean([c["hits"] for c in hc_info])),
@@ -691,6 +702,18 @@ def hc_bytes(N: int, hits: int, nscat: int, nb: int, s: int) -> float:
     diagonal sums (A and B parts), x read and y written for nb right-hand sides, one 8-byte hit
     record and one nb-wide gather per off-diagonal hit, and the amplitude table (A and B) once."""
     return N * (16 + 2 * s + 2 * s * nb) + hits * (8 + s * nb) + nscat * 2 * s
+
+
+def pair_table_bytes(info: dict, N: int) -> int:
+    """Size of the pair tables in a hit_cache_info(), which counts them beside the hit records (8 bytes
+    per hit, 64 per row); 0 where the map has the records alone."""
+    return info["bytes"] - (info["hits"] * 8 + (N + 1) * 8 + N * 56) if info["mode"] == "full" else 0
+
+
+def pair_bytes(tables: int, ne: int, N: int, s: int) -> float:
+    """Algorithmic bytes of one map application over the pair tables: the tables once, psi written and
+    read and x gathered for every pair of every row, x and y once for the diagonal."""
+    return tables + N * (ne * (ne - 1) // 2) * 3 * s + N * (8 + 2 * s)
 
 
 def block_bytes(N: int, nnz: int, nscat: int, nb: int, s: int) -> float:
@@ -779,7 +802,7 @@ def main():
     elapsed = sum(step_ms) / 1e3
     launches = _lib.kernel_launches() - launches0
     # per-launch device time of the dominant kernel: the first (up to 3) timed sectors again with
-    # per-launch events (which need eager launches: the timed steps replay captured graphs)
+    # per-launch events (which need separate launches: the timed steps are cooperative kernels)
     h.profile(True)
     hc_info = []
     for sidx, _, _ in all_vals[:3]:
@@ -1017,7 +1040,7 @@ def main():
                     "d2h_bytes_per_step": int(np.mean(d2h))},
             "gpu_launches": int(all_sum(launches, world)),
             "clocks": clk.summary(),
-            "batching": {"cuda_graphs": "restart cycles replayed as captured graphs (first cycle eager)",
+            "batching": {"step": "block map + one cooperative launch (projection, update, second pass, scaling)",
                          "block_map_autotune": tuning},
             "hit_cache": ({"hits_per_sector": float(np.mean([c["hits"] for c in hc_info])),
                            "bytes_per_sector": float(np.mean([c["bytes"] for c in hc_info])),

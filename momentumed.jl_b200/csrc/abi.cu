@@ -5,6 +5,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <vector>
@@ -231,6 +233,15 @@ void ensure_ready(momed_handle* h) {
 thread_local cudaStream_t g_alloc_stream = nullptr;
 thread_local BlockCache* g_alloc_cache = nullptr;
 
+KeptBlocks<CudaBlocks>& kept_blocks(int device) {
+    static std::mutex mu;
+    static auto* all = new std::map<int, std::unique_ptr<KeptBlocks<CudaBlocks>>>();   // handles may close at exit
+    std::lock_guard<std::mutex> lk(mu);
+    auto& k = (*all)[device];
+    if (!k) k.reset(new KeptBlocks<CudaBlocks>());
+    return *k;
+}
+
 }  // namespace momed
 
 namespace {
@@ -331,6 +342,7 @@ int momed_create(int device, momed_handle** out) {
     if (device < 0 || device >= ndev) return MOMED_EINVAL;
     momed_handle* h = new momed_handle();
     h->device = device;
+    h->blocks.kept = &kept_blocks(device);
     int rc = guarded(h, [&]() {
         keep_pool_memory(device);
         if (!take_parts(h)) {
@@ -377,7 +389,7 @@ int momed_destroy(momed_handle* h) {
     const HandleParts parts{h->device, hs, h->ev0, h->ev1};
     {
         AllocScope scope(hs);
-        h->blocks.flush(hs);
+        h->blocks.drop(hs);
         delete h;   // releases every DevBuf, ordered on the handle's stream
     }
     if (se == cudaSuccess) se = cudaStreamSynchronize(hs);
@@ -416,7 +428,7 @@ int momed_set_hbm_budget(momed_handle* h, int64_t bytes) {
     if (!h || bytes < 0) return MOMED_EINVAL;
     h->hbm_budget = bytes;
     h->blocks.on = bytes == 0;
-    if (bytes > 0) h->blocks.flush(h->stream);
+    if (bytes > 0) h->blocks.drop(h->stream);
     return MOMED_OK;
 }
 

@@ -574,11 +574,13 @@ static int cache_policy(const momed_handle* h) {
     return -1;
 }
 
-bool fits_free(const momed_handle* h, int64_t bytes, double share) {
-    if (bytes <= kSmallBytes || bytes <= (int64_t)h->blocks.held) return true;   // the latter is the handle's already
+bool fits_free(int64_t bytes, double share) {
+    if (bytes <= kSmallBytes) return true;
+    const double kept = (double)kept_blocks().held();
+    if ((double)bytes <= share * kept) return true;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
-    return (double)bytes <= share * ((double)free_b + (double)h->blocks.held);
+    return (double)bytes <= share * ((double)free_b + kept);
 }
 
 // Hit records when they fit a quarter of the free memory, else the slot mode when that fits 30%
@@ -588,8 +590,8 @@ int hit_cache_wanted(const momed_handle* h) {
     const int pol = cache_policy(h);
     if (pol == 2) return slots_ok ? 2 : 0;
     if (pol >= 0) return pol;
-    if (fits_free(h, hit_cache_bytes(h->n, h->nnz), 0.25)) return 1;
-    if (slots_ok && fits_free(h, slot_cache_bytes(h->n, h->nnz), 0.30)) return 2;
+    if (fits_free(hit_cache_bytes(h->n, h->nnz), 0.25)) return 1;
+    if (slots_ok && fits_free(slot_cache_bytes(h->n, h->nnz), 0.30)) return 2;
     return 0;
 }
 
@@ -647,7 +649,7 @@ static void build_records(momed_handle* h, int mode) {
     }
     const int64_t nnz = rp[n];
     const int64_t need = mode == 1 ? hit_cache_bytes(n, nnz) : slot_cache_bytes(n, nnz);
-    if (!fits_free(h, need, 0.9))
+    if (!fits_free(need, 0.9))
         throw Error{MOMED_ENOMEM, "hit cache: needs " + std::to_string(need) + " bytes, more than is free"};
     hc.row_ptr.resize(n + 1);
     hc.dg64.resize(2 * n);
@@ -687,7 +689,7 @@ static void build_records(momed_handle* h, int mode) {
 void build_hit_cache(momed_handle* h, int mode) {
     HitCache& hc = h->hcache;
     hc.release();
-    if (mode == 1 && pair_possible(h) && fits_free(h, pair_bytes(h), 0.9) && build_pair_cache(h)) return;
+    if (mode == 1 && pair_possible(h) && fits_free(pair_bytes(h), 0.9) && build_pair_cache(h)) return;
     build_records(h, mode);
 }
 
@@ -706,7 +708,7 @@ void ensure_hit_cache(momed_handle* h) {
         return;
     }
     if (pol && pol != 2 && !hc.pair.built && !(hc.built && hc.mode == 2) && pair_possible(h) &&
-        (pol == 1 || fits_free(h, pair_bytes(h), 0.25))) {
+        (pol == 1 || fits_free(pair_bytes(h), 0.25))) {
         try {
             build_pair_cache(h);
         } catch (const Error& e) {
@@ -733,7 +735,7 @@ void ensure_hit_records(momed_handle* h) {
     ensure_ready(h);
     int mode = 1;
     if (!hc.built) mode = hit_cache_wanted(h);
-    else if (!fits_free(h, hit_cache_bytes(h->n, hc.nnz), cache_policy(h) == 1 ? 0.9 : 0.25)) mode = 0;
+    else if (!fits_free(hit_cache_bytes(h->n, hc.nnz), cache_policy(h) == 1 ? 0.9 : 0.25)) mode = 0;
     if (!mode) return;
     try {
         build_records(h, mode);
@@ -748,7 +750,7 @@ void ensure_hit_records(momed_handle* h) {
 // hit cache, which the caller did not ask for).
 void ensure_plain_pair(momed_handle* h) {
     HitCache& hc = h->hcache;
-    if (cache_policy(h) != -1 || !pair_possible(h) || !fits_free(h, pair_bytes(h), 0.25)) return;
+    if (cache_policy(h) != -1 || !pair_possible(h) || !fits_free(pair_bytes(h), 0.25)) return;
     try {
         build_pair_map(h);
     } catch (const Error& e) {

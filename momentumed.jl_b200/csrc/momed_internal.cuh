@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/momed.h"
+#include "blockcache.h"
 
 namespace momed {
 
@@ -48,53 +49,38 @@ inline std::string base_name(const char* path) {
 // buffers does not synchronise the device and solves on other streams keep running.
 extern thread_local cudaStream_t g_alloc_stream;
 
-// Large blocks that a handle's buffers gave back, kept for its next solve.  A solve frees and
-// allocates gigabytes; from the device's pool a block freed on one stream and taken on another
-// (several handles in turn) is often not reusable yet, and the pool maps new memory instead
-// (measured: 30-70 ms of a 3x10 solve or a 32-parameter sweep, once 1.1 s).  All of a handle's
-// buffers are ordered on its one stream, so its own blocks need no event.  Held at most kMaxHeld
-// bytes; given back to the pool when an allocation is refused, when a budget is set and with the
-// handle.  Off for handles with an HBM budget and for serving slots, which account for every byte.
+struct CudaBlocks {
+    using Stream = cudaStream_t;
+    using Event = cudaEvent_t;
+    static bool create(Event& e) { return cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess; }
+    static bool record(Event e, Stream st) { return cudaEventRecord(e, st) == cudaSuccess; }
+    static bool passed(Event e) {
+        const bool yes = cudaEventQuery(e) == cudaSuccess;
+        if (!yes) cudaGetLastError();      // not ready is not an error
+        return yes;
+    }
+    static void wait(Stream st, Event e) { cudaStreamWaitEvent(st, e, 0); }
+    static void free(void* p, Stream st) { cudaFreeAsync(p, st); }
+};
+KeptBlocks<CudaBlocks>& kept_blocks(int device);     // abi.cu: one per device, never destroyed
+inline KeptBlocks<CudaBlocks>& kept_blocks() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return kept_blocks(dev);
+}
+
+// A handle's way to the device's kept blocks (its address names the owner).  Off for handles with an
+// HBM budget; serving slots run without one: both account for every byte.
 struct BlockCache {
-    static constexpr size_t kMinBlock = size_t(1) << 20;
-    static constexpr size_t kMaxHeld = size_t(16) << 30;
-    struct Block { void* p; size_t bytes; };
-    std::vector<Block> blocks;             // oldest first
-    size_t held = 0;
+    KeptBlocks<CudaBlocks>* kept = nullptr;
     bool on = true;
-    // a block of at least `bytes`, at most a quarter larger; null: none
     void* take(size_t bytes, size_t& got) {
-        size_t best = blocks.size();
-        for (size_t i = 0; i < blocks.size(); ++i)
-            if (blocks[i].bytes >= bytes && blocks[i].bytes <= bytes + bytes / 4 &&
-                (best == blocks.size() || blocks[i].bytes < blocks[best].bytes))
-                best = i;
-        if (best == blocks.size()) return nullptr;
-        void* p = blocks[best].p;
-        got = blocks[best].bytes;
-        held -= got;
-        blocks.erase(blocks.begin() + best);
-        return p;
+        if (!on || !kept || bytes < KeptBlocks<CudaBlocks>::kMinBlock) return nullptr;
+        return kept->take(bytes, this, got);
     }
-    bool put(void* p, size_t bytes, cudaStream_t st) noexcept {
-        if (!on || bytes < kMinBlock || bytes > kMaxHeld) return false;
-        try {
-            blocks.push_back({p, bytes});
-        } catch (...) {
-            return false;
-        }
-        held += bytes;
-        while (held > kMaxHeld) {
-            cudaFreeAsync(blocks.front().p, st);
-            held -= blocks.front().bytes;
-            blocks.erase(blocks.begin());
-        }
-        return true;
-    }
-    void flush(cudaStream_t st) noexcept {
-        for (const Block& b : blocks) cudaFreeAsync(b.p, st);
-        blocks.clear();
-        held = 0;
+    bool put(void* p, size_t bytes) noexcept { return on && kept && kept->put(p, bytes, this, g_alloc_stream); }
+    void drop(cudaStream_t st) noexcept {
+        if (kept) kept->drop(this, st);
     }
 };
 extern thread_local BlockCache* g_alloc_cache;
@@ -130,7 +116,7 @@ struct DevBuf {
     }
     ~DevBuf() { release(); }
     void release() {
-        if (p && !(g_alloc_cache && g_alloc_cache->put(p, cap, g_alloc_stream))) cudaFreeAsync(p, g_alloc_stream);
+        if (p && !(g_alloc_cache && g_alloc_cache->put(p, cap))) cudaFreeAsync(p, g_alloc_stream);
         p = nullptr;
         n = cap = 0;
     }
@@ -145,20 +131,18 @@ struct DevBuf {
         release();
         if (count == 0) return;
         const size_t bytes = count * sizeof(T);
-        BlockCache* const c = g_alloc_cache;
-        if (c && c->on && bytes >= BlockCache::kMinBlock) {
-            p = static_cast<T*>(c->take(bytes, cap));
-            if (p) {
-                n = count;
-                return;
-            }
+        if (g_alloc_cache) p = static_cast<T*>(g_alloc_cache->take(bytes, cap));
+        if (p) {
+            n = count;
+            return;
         }
         cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, g_alloc_stream);
-        if (e != cudaSuccess && c && c->held > 0) {        // once more with the kept blocks back in the pool
+        if (e != cudaSuccess) {            // once more with all handles' kept blocks back in the pool
             cudaGetLastError();
-            c->flush(g_alloc_stream);
-            cudaStreamSynchronize(g_alloc_stream);
-            e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, g_alloc_stream);
+            if (kept_blocks().reclaim(g_alloc_stream)) {
+                cudaStreamSynchronize(g_alloc_stream);
+                e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, g_alloc_stream);
+            }
         }
         if (e != cudaSuccess) {
             p = nullptr;
@@ -419,7 +403,7 @@ struct momed_handle {
     bool own_stream = false;
     std::string last_error;
     int64_t hbm_budget = 0;
-    momed::BlockCache blocks;              // declared before the buffers that give back to it
+    momed::BlockCache blocks;
 
     int64_t n = 0;                         // basis size
     momed::DevBuf<uint64_t> basis;
@@ -473,11 +457,11 @@ namespace momed {
 // binomial table C(n, k), n, k in [0, 32], on the device (built once per process per device)
 const uint32_t* device_binomials();
 
-// hitcache.cu: whether bytes fit the share of the free device memory (the handle's kept blocks count
-// as free).  Up to kSmallBytes, and up to what the handle has kept, nothing is asked: cudaMemGetInfo
-// took 0.1 to 14 ms
+// hitcache.cu: whether bytes fit the share of the free device memory (kept blocks count as free).  Up
+// to kSmallBytes, and up to that share of what is kept, nothing is asked: cudaMemGetInfo took 0.1 to
+// 14 ms
 constexpr int64_t kSmallBytes = 64 << 20;
-bool fits_free(const momed_handle* h, int64_t bytes, double share);
+bool fits_free(int64_t bytes, double share);
 
 // index.cu
 void build_index(momed_handle* h);

@@ -334,7 +334,7 @@ int spmv_grid(int64_t rows) {
 int64_t sparse_bytes_per_entry(bool pair) { return 4 + 16 + 8 + (pair ? 16 : 0); }
 
 static void require_room(const momed_handle* h, int64_t need) {
-    if ((h->hbm_budget > 0 && need > h->hbm_budget) || !fits_free(h, need, 0.9))
+    if ((h->hbm_budget > 0 && need > h->hbm_budget) || !fits_free(need, 0.9))
         throw Error{MOMED_ENOMEM, "sparse method: the matrix needs " + std::to_string(need) +
                                      " bytes, more than is available"};
 }

@@ -833,8 +833,9 @@ int block_size_for(momed_handle* h, int nev, int precision) {
     // FP64 refinement): two-component 4x6, nev 8: 2.73 s against 7.56 s for the mixed block solver
     // (whose FP64 phase restarts from B of the refined vectors) and 4.2 s for the FP64 one.
     // Over the pair tables the single-vector solver wins at every size: two-component 4x6, nev 8, 1.00
-    // solves/s against 0.21 with B = 4 on the hit records, 3x10, nev 6, 2.8 against 1.60.
-    if (h->hcache.pair.built && !h->hcache.records) return 0;
+    // solves/s against 0.21 with B = 4 on the hit records, 3x10, nev 6, 2.8 against 1.60 (also where a
+    // sweep has built the records before).
+    if (h->hcache.pair.built) return 0;
     if (nev < 6 || h->n < (h->hcache.full() ? 2000000 : 500000)) return 0;
     if (precision == MOMED_PREC_MIXED) return 0;
     return nev <= 10 ? 4 : 8;

@@ -291,6 +291,7 @@ struct PairPlanView {
     const int4* cls;           // [nclass] {pairs P, offset in mask/coup, offset in V, 0}
     const uint64_t* mask;      // pair masks, class by class
     const uint32_t* coup;      // per pair: the pairs of its class it is coupled to (not itself)
+    const uint32_t* listed;    // the same with itself where the list has that term
     const int32_t* ptab;       // [64 * 64] class << 8 | slot of the pair {a < b}, -1: none
 };
 struct PairPlan {
@@ -299,9 +300,10 @@ struct PairPlan {
     int64_t nv = 0;            // sum of P * P
     double density = 0.0;      // share of the off-diagonal couplings that the list has
     std::vector<int> P;        // pairs of each class
+    uint64_t has_d = 0;        // orbitals with a one-body term
     DevBuf<int4> cls;
     DevBuf<uint64_t> mask;
-    DevBuf<uint32_t> coup;
+    DevBuf<uint32_t> coup, listed;
     DevBuf<int32_t> ptab, vslot, d1;   // vslot [nv] and d1 [64]: term slots of V and the one-body diagonal
     DevBuf<double2> v64, d64;          // their values at u64 / u32
     DevBuf<float2> v32, d32;

@@ -288,14 +288,23 @@ __global__ void k_pair_values(const int32_t* __restrict__ vslot, int64_t nv, con
 }
 
 // Four chains of FMAs per output; FP32 reads V two pairs at a time (16 bytes, as FP64 does one).
+// A value is finite when its parts' high bits without their signs (top: the larger) are below kInf.
 template <typename R> struct PairV;
 template <> struct PairV<double> {
+    static constexpr int kInf = 0x7ff00000;
+    static __device__ __forceinline__ int top(double2 x) {
+        return max(__double2hiint(x.x) & 0x7fffffff, __double2hiint(x.y) & 0x7fffffff);
+    }
     static __device__ __forceinline__ double2 flip(double2 x, uint32_t sign) {
         return make_double2(__hiloint2double(__double2hiint(x.x) ^ (int)sign, __double2loint(x.x)),
                             __hiloint2double(__double2hiint(x.y) ^ (int)sign, __double2loint(x.y)));
     }
 };
 template <> struct PairV<float> {
+    static constexpr int kInf = 0x7f800000;
+    static __device__ __forceinline__ int top(float2 x) {
+        return max(__float_as_int(x.x) & 0x7fffffff, __float_as_int(x.y) & 0x7fffffff);
+    }
     static __device__ __forceinline__ float2 flip(float2 x, uint32_t sign) {
         return make_float2(__uint_as_float(__float_as_uint(x.x) ^ sign), __uint_as_float(__float_as_uint(x.y) ^ sign));
     }
@@ -393,13 +402,63 @@ k_pair_ids(PairView pv, PairPlanView pp, const typename Cx<R>::T* __restrict__ V
     else pair_ids_body<R, PM>(pv, w, P, Vs, x, psi);
 }
 
-// y[row] = sum of the psi of the row's pairs + one-body diagonal x[row]: a lane per row, G warps
-// share the pairs of 32 rows (sums combined in a fixed order).
+// y[row] term by term, for a row whose sum is not finite.  psi takes couplings that the list lacks (V = 0)
+// and pairs that a state lacks (phi = 0) along, which add nothing to finite values but spread an infinity
+// or a NaN of x or V over the class; here it stays with the rows that the list connects to it.  Rare, so
+// targets are searched in the sorted basis, and a test per row is all that the usual rows pay (48 registers
+// instead of 32: 205 -> 200 us for c128 on 1.0M states, 16.6 -> 17.6 for c64 on 174k; held to 32: 224 and
+// 20.4).  Tests in k_pair_ids cost 1 to 15% of the map, on its values, its products or once per tile.
+template <typename R>
+__device__ __noinline__ typename Cx<R>::T pair_row_apart(const PairPlanView& pp, const uint64_t* basis, int64_t n,
+                                                         int64_t row, const typename Cx<R>::T* V,
+                                                         const typename Cx<R>::T* Ds, uint64_t has_d,
+                                                         const typename Cx<R>::T* x) {
+    using C2 = typename Cx<R>::T;
+    const uint64_t s = basis[row];
+    C2 acc = cx0<R>();
+    auto add = [&](C2 c, int64_t j, bool neg) {
+        const C2 v = x[j];
+        const R pr = c.x * v.x - c.y * v.y, pi = c.x * v.y + c.y * v.x;
+        acc.x += neg ? -pr : pr;
+        acc.y += neg ? -pi : pi;
+    };
+#pragma unroll 1
+    for (uint64_t h = s; h; h &= h - 1ull) {
+        const int lo = __ffsll((long long)h) - 1;
+        if ((has_d >> lo) & 1ull) add(Ds[lo], row, false);
+#pragma unroll 1
+        for (uint64_t g = h & (h - 1ull); g; g &= g - 1ull) {
+            const int hi = __ffsll((long long)g) - 1, cs = pp.ptab[lo * 64 + hi];
+            if (cs < 0) continue;
+            const int4 cl = pp.cls[cs >> 8];
+            const int p = cs & 255;
+            const uint64_t mp = (1ull << lo) | (1ull << hi), rest = s & ~mp;
+#pragma unroll 1
+            for (uint32_t m = pp.listed[cl.y + p]; m; m &= m - 1u) {
+                const int q = __ffs((int)m) - 1;
+                const uint64_t mq = pp.mask[cl.y + q], t = rest | mq;
+                if (rest & mq) continue;
+                int64_t b = 0, e = n;
+                while (b < e) {
+                    const int64_t c = (b + e) / 2;
+                    if (basis[c] < t) b = c + 1;
+                    else e = c;
+                }
+                if (b < n && basis[b] == t)
+                    add(V[cl.z + p * cl.x + q], b, __popcll(rest & (between(mp) ^ between(mq))) & 1);
+            }
+        }
+    }
+    return acc;
+}
+
+// y[row] = sum of the psi of the row's pairs + one-body diagonal x[row] (has_d: the orbitals with a one-body
+// term): a lane per row, G warps share the pairs of 32 rows (sums combined in a fixed order).
 template <typename R>
 __global__ void __launch_bounds__(kPT)
-k_pair_rows(PairView pv, const uint64_t* __restrict__ basis, const typename Cx<R>::T* __restrict__ D,
-            const typename Cx<R>::T* __restrict__ psi, const typename Cx<R>::T* __restrict__ x,
-            typename Cx<R>::T* __restrict__ y, int G) {
+k_pair_rows(PairView pv, PairPlanView pp, const uint64_t* __restrict__ basis, const typename Cx<R>::T* __restrict__ V,
+            const typename Cx<R>::T* __restrict__ D, uint64_t has_d, const typename Cx<R>::T* __restrict__ psi,
+            const typename Cx<R>::T* __restrict__ x, typename Cx<R>::T* __restrict__ y, int G) {
     using C2 = typename Cx<R>::T;
     __shared__ C2 Ds[64];
     __shared__ C2 part[kPT];
@@ -453,7 +512,10 @@ k_pair_rows(PairView pv, const uint64_t* __restrict__ basis, const typename Cx<R
             }
         }
     }
-    if (g == 0 && row < pv.n) y[row] = acc;
+    if (g == 0 && row < pv.n) {
+        if (PairV<R>::top(acc) >= PairV<R>::kInf) acc = pair_row_apart<R>(pp, basis, pv.n, row, V, Ds, has_d, x);
+        y[row] = acc;
+    }
 }
 
 int pair_sms() {
@@ -479,6 +541,7 @@ PairPlanView PairPlan::view() const {
     v.cls = cls.p;
     v.mask = mask.p;
     v.coup = coup.p;
+    v.listed = listed.p;
     v.ptab = ptab.p;
     return v;
 }
@@ -557,7 +620,7 @@ bool pair_plan(momed_handle* h) {
         pmax = std::max(pmax, P[c]);
     }
     std::vector<uint64_t> mask(np);
-    std::vector<uint32_t> coup(np, 0u);
+    std::vector<uint32_t> coup(np, 0u), listed(np, 0u);
     std::vector<int32_t> ptab(64 * 64, -1), vslot(voff, -1);
     for (int i = 0; i < np; ++i) {
         mask[cls[cls_of[i]].y + slot_of[i]] = pairs[i];
@@ -570,6 +633,7 @@ bool pair_plan(momed_handle* h) {
             const int o = at(tout[t]), i = at(tin[t]);
             const int4 c = cls[cls_of[o]];
             vslot[c.z + slot_of[o] * c.x + slot_of[i]] = (int32_t)t;
+            listed[c.y + slot_of[o]] |= 1u << slot_of[i];
             if (o != i) {
                 coup[c.y + slot_of[o]] |= 1u << slot_of[i];
                 ++ncoup;
@@ -579,11 +643,15 @@ bool pair_plan(momed_handle* h) {
     upload(pl.cls, cls, st);
     upload(pl.mask, mask, st);
     upload(pl.coup, coup, st);
+    upload(pl.listed, listed, st);
     upload(pl.ptab, ptab, st);
     upload(pl.vslot, vslot, st);
     upload(pl.d1, d1, st);
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
     pl.P = P;
+    pl.has_d = 0;
+    for (int o = 0; o < 64; ++o)
+        if (d1[o] >= 0) pl.has_d |= 1ull << o;
     pl.nclass = nc;
     pl.pmax = pmax;
     pl.nv = voff;
@@ -801,7 +869,8 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
     int G = 1;
     while (G < 8 && rw * G < want) G *= 2;
     const int per = kPT / 32 / G;
-    k_pair_rows<R><<<(unsigned)((rw + per - 1) / per), kPT, 0, st>>>(pm.view(), h->basis.p, D.p, psi, x, y, G);
+    k_pair_rows<R><<<(unsigned)((rw + per - 1) / per), kPT, 0, st>>>(pm.view(), pl.view(), h->basis.p, V.p, D.p, pl.has_d, psi, x,
+                                                                     y, G);
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
 }

@@ -390,8 +390,10 @@ struct BlockLanczos {
     // replay them, stay for per-launch timing and MOMED_COOP=0.
     bool coopb = false;
     BlockStepBufs<VT> bs;
-    // set on the device by a cooperative step whose grid barrier gave up; none with the separate kernels
+    // set on the device by a cooperative step whose grid barrier gave up; none with the separate kernels.
+    // Column k, from which the steps went, is as it was then: they run once more after separate().
     const int* err_flag() const { return coop ? cy.a.err : coopb ? bs.a.err : nullptr; }
+    void separate() { coop = coopb = false; }
 
     ~BlockLanczos() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
@@ -441,8 +443,7 @@ struct BlockLanczos {
             const char* e = std::getenv("MOMED_GRAPHS");
             use_graphs = !(e && e[0] == '0') && !hh->prof;   // per-launch timing needs eager launches
         }
-        const char* ce = std::getenv("MOMED_COOP");
-        const bool any_coop = !(ce && ce[0] == '0') && !hh->prof;
+        const bool any_coop = coop_switch() != COOP_OFF && !hh->prof;
         const bool want_coop = NB == 1 && any_coop && !hh->sparse.built && hh->hcache.pair.built;
         {   // kernel attributes are set before any capture
             constexpr size_t smem_max = (size_t)kMaxCols * NB * sizeof(double2);
@@ -463,7 +464,7 @@ struct BlockLanczos {
         beta.resize((size_t)NB * m);
         flag.resize(NB);
         any.resize(1);
-        if (want_coop && cy.prepare(N, false, alpha.p, beta.p, dgks, st)) {
+        if (want_coop && cy.prepare(N, CYCLE_NONE, alpha.p, beta.p, dgks, st)) {
             coop = true;
             use_graphs = false;
         } else if (any_coop && bs.prepare(N, NB, m, alpha.p, beta.p, st)) {
@@ -534,13 +535,10 @@ struct BlockLanczos {
         BlockMv<VT>::run(h, col(j), w, ud.p, NB, u0);   // counted by its launcher
         if (coop) {
             cy.a.keep = dgks;
-            cy.steps(V.p, j, j + 1, CYCLE_NONE, st);
-            return;
+            if (cy.steps(V.p, j, j + 1, st)) return;
         }
-        if (coopb) {
-            bs.step(V.p, j, dgks, st);
-            return;
-        }
+        if (coopb && bs.step(V.p, j, dgks, st)) return;
+        separate();                  // not planned, or refused
         const int nc = j + 1;
         proj(nc, w, coefA.p, nullptr);
         update(nc, coefA.p, w, nullptr, nullptr);
@@ -606,17 +604,20 @@ struct BlockLanczos {
         std::vector<int> nconv(NB, 0);
         out.broken.assign(NB, 0);
         for (;;) {
-            if (restarts == 0) {
-                for (int j = k; j < m; ++j) { step(j); ++steps; }
-            } else {
-                cycle(k, steps);
+            for (;;) {
+                if (restarts == 0) {
+                    for (int j = k; j < m; ++j) { step(j); ++steps; }
+                } else {
+                    cycle(k, steps);
+                }
+                MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
+                MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
+                int err = 0;
+                if (const int* e = err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));
+                MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+                if (!err) break;
+                separate();
             }
-            MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
-            MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
-            int err = 0;
-            if (const int* e = err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));
-            MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-            CycleBufs<VT>::check(err);
             // per right-hand side projected eigenproblems, in parallel on the host
             auto solve_r = [&](int r) {
                 std::vector<double> T((size_t)m * m, 0.0);
@@ -1022,33 +1023,35 @@ int run_batch(momed_handle* h, const momed_solve_opts* o, const double* u, int32
                 note_launches(2);
                 MOMED_CUDA_TRY(cudaGetLastError());
                 LR.orth_start(k1);
-                for (int j = k1; j < m; ++j) LR.step(j);
-                matvecs += (int64_t)p * nu;
                 std::vector<double> ha((size_t)NB * m), hb((size_t)NB * m);
-                MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), LR.alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
-                MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), LR.beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
-                // FP64 Gram blocks: b_a^H H b_i and b_a^H b_i for the anchors i against [X, Q]
                 std::vector<std::vector<std::complex<double>>> G(NB, std::vector<std::complex<double>>((size_t)d * d)),
                     S(NB, std::vector<std::complex<double>>((size_t)d * d));
-                // FP64 Gram blocks: b_a^H H b_i and b_a^H b_i for the anchors i against [X, Q]; the
-                // 2 k1 right-hand sides (W_i, then X_i) go kGramRhs at a time
                 const int nrhs = 2 * k1;
-                for (int g0 = 0; g0 < nrhs; g0 += kGramRhs) {
-                    const int nr = std::min(kGramRhs, nrhs - g0);
-                    const double2* rhs[kGramRhs];
-                    for (int j = 0; j < nr; ++j)
-                        rhs[j] = g0 + j < k1 ? Wb.p + (size_t)(g0 + j) * stride : Xb.p + (size_t)(g0 + j - k1) * stride;
-                    block_gram(Xb.p, N, NB, k1, rhs, nr, gpart.p, gx.p + (size_t)g0 * k1 * NB, st);     // x_a^H rhs
-                    block_gram(LR.col(k1), N, NB, p, rhs, nr, gpart.p, gq.p + (size_t)g0 * p * NB, st); // q_j^H rhs
-                    note_launches(4);
-                }
-                int err = 0;
-                if (const int* e = LR.err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));
                 std::vector<double2> hx((size_t)gx_n), hq((size_t)gq_n);
-                MOMED_CUDA_TRY(cudaMemcpyAsync(hx.data(), gx.p, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
-                MOMED_CUDA_TRY(cudaMemcpyAsync(hq.data(), gq.p, hq.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
-                MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-                CycleBufs<float2>::check(err);
+                for (;;) {
+                    for (int j = k1; j < m; ++j) LR.step(j);
+                    matvecs += (int64_t)p * nu;
+                    MOMED_CUDA_TRY(cudaMemcpyAsync(ha.data(), LR.alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, st));
+                    MOMED_CUDA_TRY(cudaMemcpyAsync(hb.data(), LR.beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, st));
+                    // FP64 Gram blocks: b_a^H H b_i and b_a^H b_i for the anchors i against [X, Q]; the
+                    // 2 k1 right-hand sides (W_i, then X_i) go kGramRhs at a time
+                    for (int g0 = 0; g0 < nrhs; g0 += kGramRhs) {
+                        const int nr = std::min(kGramRhs, nrhs - g0);
+                        const double2* rhs[kGramRhs];
+                        for (int j = 0; j < nr; ++j)
+                            rhs[j] = g0 + j < k1 ? Wb.p + (size_t)(g0 + j) * stride : Xb.p + (size_t)(g0 + j - k1) * stride;
+                        block_gram(Xb.p, N, NB, k1, rhs, nr, gpart.p, gx.p + (size_t)g0 * k1 * NB, st);     // x_a^H rhs
+                        block_gram(LR.col(k1), N, NB, p, rhs, nr, gpart.p, gq.p + (size_t)g0 * p * NB, st); // q_j^H rhs
+                        note_launches(4);
+                    }
+                    int err = 0;
+                    if (const int* e = LR.err_flag()) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, e, sizeof(int), cudaMemcpyDeviceToHost, st));
+                    MOMED_CUDA_TRY(cudaMemcpyAsync(hx.data(), gx.p, hx.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
+                    MOMED_CUDA_TRY(cudaMemcpyAsync(hq.data(), gq.p, hq.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
+                    MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+                    if (!err) break;
+                    LR.separate();
+                }
                 for (int jr = 0; jr < nrhs; ++jr) {
                     const int i = jr < k1 ? jr : jr - k1;
                     auto& M = jr < k1 ? G : S;

@@ -430,15 +430,14 @@ bool block_step_plan(int64_t N, int nb, int m, BlockStepArgs<VT>& a, int& grid) 
 }
 
 template <typename VT>
-void launch_block_step(const BlockStepArgs<VT>& a, int nb, int grid, cudaStream_t st) {
+bool launch_block_step(const BlockStepArgs<VT>& a, int nb, int grid, cudaStream_t st) {
     void* args[] = {const_cast<BlockStepArgs<VT>*>(&a)};
-    MOMED_CUDA_TRY(cudaLaunchCooperativeKernel(step_kernel<VT>(nb), dim3(grid), dim3(kBT), args, step_smem<VT>(nb, a.m), st));
-    note_launches(1);
+    return launch_cooperative(step_kernel<VT>(nb), grid, kBT, args, step_smem<VT>(nb, a.m), st);
 }
 
 template bool block_step_plan<double2>(int64_t, int, int, BlockStepArgs<double2>&, int&);
 template bool block_step_plan<float2>(int64_t, int, int, BlockStepArgs<float2>&, int&);
-template void launch_block_step<double2>(const BlockStepArgs<double2>&, int, int, cudaStream_t);
-template void launch_block_step<float2>(const BlockStepArgs<float2>&, int, int, cudaStream_t);
+template bool launch_block_step<double2>(const BlockStepArgs<double2>&, int, int, cudaStream_t);
+template bool launch_block_step<float2>(const BlockStepArgs<float2>&, int, int, cudaStream_t);
 
 }  // namespace momed

@@ -47,7 +47,7 @@ template <typename VT> struct BlockStepArgs {
 
 // Rows per block and the grid for bases of m + 1 columns; false where a launch cannot be resident.
 template <typename VT> bool block_step_plan(int64_t N, int nb, int m, BlockStepArgs<VT>& a, int& grid);
-template <typename VT> void launch_block_step(const BlockStepArgs<VT>& a, int nb, int grid, cudaStream_t st);
+template <typename VT> bool launch_block_step(const BlockStepArgs<VT>& a, int nb, int grid, cudaStream_t st);
 
 template <typename VT> struct BlockStepBufs {
     BlockStepArgs<VT> a{};
@@ -61,8 +61,8 @@ template <typename VT> struct BlockStepBufs {
         part.resize((size_t)grid * (m + 1) * nb);
         coef.resize((size_t)(m + 1) * nb);
         npart.resize((size_t)grid * nb);
-        bar.resize(3);                   // barrier, its exits, the error flag
-        MOMED_CUDA_TRY(cudaMemsetAsync(bar.p, 0, 3 * sizeof(unsigned), st));
+        bar.resize(3);
+        clear_barrier(bar.p, st);
         a.m = m;
         a.part = part.p;
         a.coef = coef.p;
@@ -73,11 +73,12 @@ template <typename VT> struct BlockStepBufs {
         a.err = reinterpret_cast<int*>(bar.p + 2);
         return true;
     }
-    void step(VT* V, int j, double keep, cudaStream_t st) {
+    // false: refused, nothing was done
+    bool step(VT* V, int j, double keep, cudaStream_t st) {
         a.V = V;
         a.j = j;
         a.keep = keep;
-        launch_block_step(a, nb, grid, st);
+        return launch_block_step(a, nb, grid, st);
     }
 };
 

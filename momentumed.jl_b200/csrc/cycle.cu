@@ -311,9 +311,17 @@ size_t cycle_smem(int rows, int chunks, size_t elem) {
 
 }  // namespace
 
+template <typename VT> static const void* cycle_kernel(int map) {
+    if constexpr (std::is_same<VT, double2>::value) {
+        if (map == CYCLE_HITS) return reinterpret_cast<const void*>(k_lanczos_cycle<double2, CYCLE_HITS>);
+        if (map == CYCLE_CSR) return reinterpret_cast<const void*>(k_lanczos_cycle<double2, CYCLE_CSR>);
+    }
+    return reinterpret_cast<const void*>(k_lanczos_cycle<VT, CYCLE_NONE>);
+}
+
 // Small sectors take at least 32 rows a block (a barrier over few blocks is shorter).
 template <typename VT>
-bool cycle_plan(int64_t N, CycleArgs<VT>& a, int& grid) {
+bool cycle_plan(int64_t N, int map, CycleArgs<VT>& a, int& grid) {
     const int sms = cycle_sms();
     if (N < 1 || sms < 1) return false;
     const int64_t rows = std::max<int64_t>(32, (N + sms - 1) / sms);
@@ -323,31 +331,25 @@ bool cycle_plan(int64_t N, CycleArgs<VT>& a, int& grid) {
     a.chunks = (int)std::min<int64_t>(kMaxChunks, std::max<int64_t>(1, rows / 128));
     a.split = rows <= 512 ? 4 : rows <= 2048 ? 2 : 1;
     grid = (int)((N + rows - 1) / rows);
-    return cycle_smem(a.rows, a.chunks, sizeof(VT)) <= kMaxSmem;
+    const size_t smem = cycle_smem(a.rows, a.chunks, sizeof(VT));
+    if (smem > kMaxSmem) return false;
+    // process-wide attribute: always the largest size, so concurrent callers never lower it
+    const void* k = cycle_kernel<VT>(map);
+    int per = 0;
+    MOMED_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    MOMED_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kCT, smem));
+    return per >= 1;
 }
 
 template <typename VT>
-void launch_cycle(CycleArgs<VT>& a, int map, int grid, cudaStream_t st) {
-    const size_t smem = cycle_smem(a.rows, a.chunks, sizeof(VT));
+bool launch_cycle(CycleArgs<VT>& a, int map, int grid, cudaStream_t st) {
     void* args[] = {&a};
-    auto go = [&](auto k) {
-        // process-wide attribute: always the largest size, so concurrent callers never lower it
-        MOMED_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-        MOMED_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(grid), dim3(kCT), args, smem, st));
-    };
-    if constexpr (std::is_same<VT, double2>::value) {
-        if (map == CYCLE_HITS) go(k_lanczos_cycle<double2, CYCLE_HITS>);
-        else if (map == CYCLE_CSR) go(k_lanczos_cycle<double2, CYCLE_CSR>);
-        else go(k_lanczos_cycle<double2, CYCLE_NONE>);
-    } else {
-        go(k_lanczos_cycle<float2, CYCLE_NONE>);
-    }
-    note_launches(1);
+    return launch_cooperative(cycle_kernel<VT>(map), grid, kCT, args, cycle_smem(a.rows, a.chunks, sizeof(VT)), st);
 }
 
-template bool cycle_plan<double2>(int64_t, CycleArgs<double2>&, int&);
-template bool cycle_plan<float2>(int64_t, CycleArgs<float2>&, int&);
-template void launch_cycle<double2>(CycleArgs<double2>&, int, int, cudaStream_t);
-template void launch_cycle<float2>(CycleArgs<float2>&, int, int, cudaStream_t);
+template bool cycle_plan<double2>(int64_t, int, CycleArgs<double2>&, int&);
+template bool cycle_plan<float2>(int64_t, int, CycleArgs<float2>&, int&);
+template bool launch_cycle<double2>(CycleArgs<double2>&, int, int, cudaStream_t);
+template bool launch_cycle<float2>(CycleArgs<float2>&, int, int, cudaStream_t);
 
 }  // namespace momed

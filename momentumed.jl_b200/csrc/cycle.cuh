@@ -1,6 +1,8 @@
 // Cooperative kernels for Lanczos steps: a single-vector cycle (cycle.cu), a step of the lockstep block
 // solver (blockstep.cu).
 #pragma once
+#include <cstdlib>
+
 #include "vecops.cuh"
 
 namespace momed {
@@ -77,25 +79,56 @@ template <typename VT> struct CycleArgs {
     const double2* val;
 };
 
+// Cooperative steps have the separate kernels to fall back on: a plan that does not fit, a launch that the
+// driver refuses (fewer SMs for this process than the device has) and a grid barrier that gave up all end
+// there, the last with the steps since the basis was last whole run again.  MOMED_COOP=0 starts there;
+// =2 and =3 make every launch give up or be refused (tests).
+enum CoopSwitch : int { COOP_OFF = 0, COOP_ON = 1, COOP_GIVES_UP = 2, COOP_REFUSED = 3 };
+inline CoopSwitch coop_switch() {
+    const char* e = std::getenv("MOMED_COOP");
+    return e && (e[0] == '0' || e[0] == '2' || e[0] == '3') ? (CoopSwitch)(e[0] - '0') : COOP_ON;
+}
+
+// A cooperative launch, counted; false when the driver cannot hold the grid at once.
+inline bool launch_cooperative(const void* k, int grid, int threads, void** args, size_t smem, cudaStream_t st) {
+    const cudaError_t e = coop_switch() == COOP_REFUSED
+                              ? cudaErrorCooperativeLaunchTooLarge
+                              : cudaLaunchCooperativeKernel(k, dim3(grid), dim3(threads), args, smem, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        cudaGetLastError();
+        return false;
+    }
+    MOMED_CUDA_TRY(e);
+    note_launches(1);
+    return true;
+}
+
+// the barrier, its exits and the error flag of a solve's launches
+inline void clear_barrier(unsigned* bar, cudaStream_t st) {
+    MOMED_CUDA_TRY(cudaMemsetAsync(bar, 0, 3 * sizeof(unsigned), st));
+    if (coop_switch() == COOP_GIVES_UP) MOMED_CUDA_TRY(cudaMemsetAsync(bar + 2, 1, sizeof(unsigned), st));
+}
+
 // Rows per block and the split of a block's work; false where a block's part of w does not fit.
-template <typename VT> bool cycle_plan(int64_t N, CycleArgs<VT>& a, int& grid);
-template <typename VT> void launch_cycle(CycleArgs<VT>& a, int map, int grid, cudaStream_t st);
+template <typename VT> bool cycle_plan(int64_t N, int map, CycleArgs<VT>& a, int& grid);
+template <typename VT> bool launch_cycle(CycleArgs<VT>& a, int map, int grid, cudaStream_t st);
 
 // The buffers of a solve's launches (partial sums, barrier) beside those the solver owns.
 template <typename VT> struct CycleBufs {
     CycleArgs<VT> a{};
-    int grid = 0;
+    int grid = 0, map = CYCLE_NONE;
     DevBuf<double2> part, xbuf;
     DevBuf<double> npart;
     DevBuf<unsigned> bar;
     // false: the solver runs its separate kernels
-    bool prepare(int64_t N, bool with_map, double* alpha, double* beta, double keep, cudaStream_t st) {
-        if (!cycle_plan(N, a, grid)) return false;
+    bool prepare(int64_t N, int kind, double* alpha, double* beta, double keep, cudaStream_t st) {
+        if (!cycle_plan(N, kind, a, grid)) return false;
+        map = kind;
         part.resize((size_t)grid * (kMaxCols + 1));
         npart.resize(grid);
-        bar.resize(3);                   // barrier, its exits, the error flag
-        MOMED_CUDA_TRY(cudaMemsetAsync(bar.p, 0, 3 * sizeof(unsigned), st));
-        if (with_map) xbuf.resize((size_t)2 * N);
+        bar.resize(3);
+        clear_barrier(bar.p, st);
+        if (map != CYCLE_NONE) xbuf.resize((size_t)2 * N);
         a.part = part.p;
         a.npart = npart.p;
         a.xbuf = xbuf.p;
@@ -106,15 +139,12 @@ template <typename VT> struct CycleBufs {
         a.err = reinterpret_cast<int*>(bar.p + 2);
         return true;
     }
-    void steps(VT* V, int j0, int j1, int map, cudaStream_t st) {
+    // false: refused, nothing was done
+    bool steps(VT* V, int j0, int j1, cudaStream_t st) {
         a.V = V;
         a.j0 = j0;
         a.j1 = j1;
-        launch_cycle(a, map, grid, st);
-    }
-    // after a synchronisation of the copy of err: a barrier that gave up ends the solve
-    static void check(int err) {
-        if (err) throw Error{MOMED_ETIMEOUT, "Lanczos cycle: a grid barrier gave up"};
+        return launch_cycle(a, map, grid, st);
     }
 };
 

@@ -135,13 +135,12 @@ struct Lanczos {
     // The map inside the cooperative kernel: CSR and hit records.  Beside the pair map each step's
     // orthogonalisation runs as one.  Candidate and slot-mode maps keep the separate kernels.
     void plan_coop() {
-        const char* e = std::getenv("MOMED_COOP");
-        if ((e && e[0] == '0') || h->prof) return;
+        if (coop_switch() == COOP_OFF || h->prof) return;
         if (h->sparse.built) coop = CYCLE_CSR;
         else if (h->hcache.pair.built) coop = CYCLE_NONE;
         else if (h->hcache.full()) coop = CYCLE_HITS;
         if (coop < 0) return;
-        if (!cy.prepare(N, coop != CYCLE_NONE, alpha, beta, 0.1, st)) {     // k_decide's share
+        if (!cy.prepare(N, coop, alpha, beta, 0.1, st)) {     // k_decide's share
             coop = -1;
             return;
         }
@@ -160,27 +159,37 @@ struct Lanczos {
             a.amp = hit_amplitudes_c128(h, st);
         }
     }
-    void coop_steps(int j0, int j1) {
-        if constexpr (std::is_same<VT, double2>::value) cy.steps(V.p, j0, j1, coop, st);
+    // false: refused, and the separate kernels from here on
+    bool coop_steps(int j0, int j1) {
+        if constexpr (std::is_same<VT, double2>::value) {
+            if (cy.steps(V.p, j0, j1, st)) return true;
+        }
+        coop = -1;
+        return false;
     }
     // steps [j0, j1)
     void steps(int j0, int j1) {
-        if (coop > CYCLE_NONE && j1 > j0) {
-            coop_steps(j0, j1);
-            return;
-        }
+        if (coop > CYCLE_NONE && j1 > j0 && coop_steps(j0, j1)) return;
         for (int j = j0; j < j1; ++j) step(j);
     }
-    // alpha and beta on the host; a barrier that gave up ends the solve
-    void fetch(double* ha, double* hb) {
-        int err = 0;
+    // Steps [j0, m), their alpha and beta on the host; returns the maps applied.  A barrier that gave up
+    // leaves column j0 as it was: the steps run once more as separate kernels, which the solve then keeps.
+    int64_t cycle(int j0, double* ha, double* hb) {
+        int64_t maps = 0;
         std::vector<double> t((size_t)2 * m);
-        MOMED_CUDA_TRY(cudaMemcpyAsync(t.data(), ab.p, t.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-        if (coop >= 0) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        MOMED_CUDA_TRY(cudaStreamSynchronize(st));
-        CycleBufs<double2>::check(err);
+        for (;;) {
+            int err = 0;
+            steps(j0, m);
+            maps += m - j0;
+            MOMED_CUDA_TRY(cudaMemcpyAsync(t.data(), ab.p, t.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+            if (coop >= 0) MOMED_CUDA_TRY(cudaMemcpyAsync(&err, cy.a.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            MOMED_CUDA_TRY(cudaStreamSynchronize(st));
+            if (!err) break;
+            coop = -1;
+        }
         std::copy(t.begin(), t.begin() + m, ha);
         std::copy(t.begin() + m, t.end(), hb);
+        return maps;
     }
 
     void normalize(VT* v) {
@@ -202,10 +211,7 @@ struct Lanczos {
     void step(int j) {
         VT* w = col(j + 1);
         apply_h(h, col(j), w);
-        if (coop == CYCLE_NONE) {
-            coop_steps(j, j + 1);
-            return;
-        }
+        if (coop == CYCLE_NONE && coop_steps(j, j + 1)) return;
         const int nc = j + 1;
         vec_proj<VT>(V.p, N, nc, w, partial.p, grid, nullptr, st);
         vec_reduce(partial.p, grid, nc + 1, coefA.p, nullptr, st);
@@ -235,9 +241,7 @@ struct Lanczos {
         for (;;) {
             int jstart = k;
             int mm = m;
-            steps(jstart, m);
-            matvecs += m - jstart;
-            fetch(ha.data(), hb.data());
+            matvecs += cycle(jstart, ha.data(), hb.data());
             // invariant-subspace breakdown inside the cycle
             double scale = 0.0;
             for (int j = k; j < m; ++j) scale = std::max(scale, std::fabs(ha[j]));
@@ -251,9 +255,7 @@ struct Lanczos {
                     hb[j] = 0.0;
                     double zero = 0.0;
                     MOMED_CUDA_TRY(cudaMemcpyAsync(beta + j, &zero, sizeof(double), cudaMemcpyHostToDevice, st));
-                    steps(j + 1, m);
-                    matvecs += m - j - 1;
-                    fetch(ha.data(), hb.data());
+                    matvecs += cycle(j + 1, ha.data(), hb.data());
                     hb[j] = 0.0;
                 }
             }
@@ -313,7 +315,7 @@ struct Lanczos {
             arrow.resize(keep);
             for (int i = 0; i < keep; ++i) arrow[i] = beta_last * U[(size_t)(m - 1) * m + i];
             k = keep;
-            ++restarts;                      // Uc is written again after the next fetch
+            ++restarts;                      // Uc is written again after the next cycle's copy
         }
     }
 };

@@ -580,7 +580,7 @@ def run_plain_workload(args, rank, world, local):
         if use_hc:
             hc = h.build_hit_cache()
             hc_info.append(hc)
-            pairs = 0 if bsz else pair_table_bytes(hc, len(sectors[sidx][1]))
+            pairs = 0 if bsz else pair_table_bytes(hc, sum(w["N_each"]), len(sectors[sidx][1]))
             nb.append(pair_bytes(pairs, sum(w["N_each"]), len(sectors[sidx][1]), 16) if pairs > 0 else
                       hc_bytes(len(sectors[sidx][1]), hc["hits"], len(pair[0]), max(bsz, 1), 16))
             nnz_mean.append(st["nnz"])
@@ -704,10 +704,11 @@ def hc_bytes(N: int, hits: int, nscat: int, nb: int, s: int) -> float:
     return N * (16 + 2 * s + 2 * s * nb) + hits * (8 + s * nb) + nscat * 2 * s
 
 
-def pair_table_bytes(info: dict, N: int) -> int:
-    """Size of the pair tables in a hit_cache_info(), which counts them beside the hit records (8 bytes
-    per hit, 64 per row); 0 where the map has the records alone."""
-    return info["bytes"] - (info["hits"] * 8 + (N + 1) * 8 + N * 56) if info["mode"] == "full" else 0
+def pair_table_bytes(info: dict, ne: int, N: int) -> int:
+    """Size of the pair tables of a freshly built cache, which has them with a workspace of 16 bytes for
+    every pair of every row, or the hit records (8 bytes per hit, 64 per row); 0 for those."""
+    records = info["hits"] * 8 + (N + 1) * 8 + N * 56
+    return info["bytes"] - N * (ne * (ne - 1) // 2) * 16 if info["mode"] == "full" and info["bytes"] != records else 0
 
 
 def pair_bytes(tables: int, ne: int, N: int, s: int) -> float:

@@ -283,8 +283,8 @@ MOMED_API int  momed_block_tuning(momed_handle* h, int32_t nb, int32_t precision
  * (MOMED_HITCACHE=0: never, =1: full whatever its size, =2: slot mode); momed_build_hit_cache builds
  * it on request (the slot mode under MOMED_HITCACHE=2; MOMED_ENOMEM when it does not fit,
  * MOMED_ESTATE while a sparse matrix is built).  hits counts the off-diagonal hits; bytes is the
- * device memory of the cache, the records of later block maps included.  momed_matvec builds the
- * pair tables by itself at the second call on a basis and operator (same memory rule; not reported
+ * device memory that the cache holds: the pair tables with their workspace, the records once they
+ * are built.  momed_matvec builds the pair tables by itself at the second call on a basis and operator (same memory rule; not reported
  * as a hit cache).  The cache is dropped with the basis, the operator, a sparse-matrix build, or
  * new amplitudes of a parametrised operator.  No reference counterpart: the reference map evaluates
  * every term at every application (ka_linearmap_kernel!,

@@ -606,11 +606,14 @@ int64_t full_cache_bytes(momed_handle* h, bool block_maps) {
 static bool build_pair_cache(momed_handle* h) {
     HitCache& hc = h->hcache;
     const auto t0 = std::chrono::steady_clock::now();
-    if (!hc.pair.built && !build_pair_map(h)) return false;
+    if (!hc.pair.built) {
+        if (!build_pair_map(h)) return false;
+        if (hc.built) hc.bytes += hc.pair.bytes;
+    }
     if (hc.built) return true;                  // beside records built before
     hc.mode = 1;
     hc.nnz = hc.pair.hits;
-    hc.bytes = hc.pair.bytes + hit_cache_bytes(h->n, hc.nnz);   // with the records of later block maps
+    hc.bytes = hc.pair.bytes;
     hc.build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     hc.built = true;
     return true;
@@ -741,8 +744,12 @@ void ensure_hit_records(momed_handle* h) {
         build_records(h, mode);
     } catch (const Error& e) {
         if (e.code != MOMED_ENOMEM) throw;
-        if (!hc.pair.built) hc.release();
-        else hc.release_records();
+        if (!hc.pair.built) {
+            hc.release();
+        } else {
+            hc.release_records();
+            hc.bytes = hc.pair.bytes;
+        }
     }
 }
 

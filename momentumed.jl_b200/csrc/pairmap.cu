@@ -790,7 +790,7 @@ bool build_pair_map(momed_handle* h) {
     pm.entries = (int64_t)th[0];
     pm.psi.resize(std::max<int64_t>(pm.entries, 1));   // here, so that the first product does not wait for it
     pm.hits = (int64_t)th[1];
-    pm.bytes = nent * 4 + slots * 4 + tiles * 16;
+    pm.bytes = (int64_t)(pm.work.bytes() + pm.tile.bytes() + pm.ent_row.bytes() + pm.row_ent.bytes() + pm.psi.bytes());
     pm.built = true;
     return true;
 }

@@ -603,11 +603,11 @@ int64_t full_cache_bytes(momed_handle* h, bool block_maps) {
 }
 
 // The pair tables as a full cache (no hit records yet).  False: declined.
-static bool build_pair_cache(momed_handle* h) {
+static bool build_pair_cache(momed_handle* h, double share) {
     HitCache& hc = h->hcache;
     const auto t0 = std::chrono::steady_clock::now();
     if (!hc.pair.built) {
-        if (!build_pair_map(h)) return false;
+        if (!build_pair_map(h, share)) return false;
         if (hc.built) hc.bytes += hc.pair.bytes;
     }
     if (hc.built) return true;                  // beside records built before
@@ -689,10 +689,10 @@ static void build_records(momed_handle* h, int mode) {
     hc.built = true;
 }
 
-void build_hit_cache(momed_handle* h, int mode) {
+void build_hit_cache(momed_handle* h, int mode, double share) {
     HitCache& hc = h->hcache;
     hc.release();
-    if (mode == 1 && pair_possible(h) && fits_free(pair_bytes(h), 0.9) && build_pair_cache(h)) return;
+    if (mode == 1 && pair_possible(h) && fits_free(pair_bytes(h), 0.9) && build_pair_cache(h, share)) return;
     build_records(h, mode);
 }
 
@@ -707,13 +707,13 @@ void ensure_hit_cache(momed_handle* h) {
     HitCache& hc = h->hcache;
     const int pol = cache_policy(h);
     if (hc.pair.built && !hc.built && pol) {      // built for momed_matvec: it serves the solver too
-        build_pair_cache(h);
+        build_pair_cache(h, 0.25);
         return;
     }
     if (pol && pol != 2 && !hc.pair.built && !(hc.built && hc.mode == 2) && pair_possible(h) &&
         (pol == 1 || fits_free(pair_bytes(h), 0.25))) {
         try {
-            build_pair_cache(h);
+            build_pair_cache(h, pol == 1 ? 0.9 : 0.25);
         } catch (const Error& e) {
             if (e.code != MOMED_ENOMEM) throw;
             hc.pair.release();
@@ -759,7 +759,7 @@ void ensure_plain_pair(momed_handle* h) {
     HitCache& hc = h->hcache;
     if (cache_policy(h) != -1 || !pair_possible(h) || !fits_free(pair_bytes(h), 0.25)) return;
     try {
-        build_pair_map(h);
+        build_pair_map(h, 0.25);
     } catch (const Error& e) {
         if (e.code != MOMED_ENOMEM) throw;
         hc.pair.release();

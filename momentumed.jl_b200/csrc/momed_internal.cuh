@@ -476,7 +476,9 @@ int64_t validate_operator(momed_handle* h);   // counts (row, term) targets miss
 int64_t hit_cache_bytes(int64_t n, int64_t hits);
 int64_t slot_cache_bytes(int64_t n, int64_t hits);
 int hit_cache_wanted(const momed_handle* h);             // 0 none, 1 full, 2 term slots only
-void build_hit_cache(momed_handle* h, int mode = 1);     // mode 1: pair tables where possible, else records
+// mode 1: pair tables where possible, else records; share: of the free memory, for what the tables take
+// beyond pair_bytes when they are counted
+void build_hit_cache(momed_handle* h, int mode = 1, double share = 0.9);
 void ensure_hit_cache(momed_handle* h);
 void build_hit_records(momed_handle* h);                 // the records of a built full cache, if missing
 void ensure_hit_records(momed_handle* h);                // before block maps: under the automatic size rule
@@ -494,8 +496,10 @@ void launch_block_hc_c128(const momed_handle* h, const double2* x, double2* y, c
 
 // pairmap.cu
 bool pair_possible(momed_handle* h);           // operator and basis take the pair form
-int64_t pair_bytes(const momed_handle* h);     // its device memory, FP64 workspace included
-bool build_pair_map(momed_handle* h);          // false: declined
+int64_t pair_bytes(const momed_handle* h);     // device memory to admit it by: the tables, the workspace, the build
+// False: declined, for the states, or because it takes more than pair_bytes when they are counted and that
+// does not fit the share of the free memory (0: pair_bytes is all there is).
+bool build_pair_map(momed_handle* h, double share);
 void launch_pair_c128(momed_handle* h, const double2* x, double2* y, double u, cudaStream_t st);
 void launch_pair_c64(momed_handle* h, const float2* x, float2* y, double u, cudaStream_t st);
 

@@ -667,9 +667,10 @@ static int64_t pairs_per_row(const momed_handle* h) {
     return ne * (ne - 1) / 2;
 }
 
-// Device memory of the tables and the FP64 workspace: row_ent and psi per (row, pair), ent_row per
-// slot (a tile has at most about twice as many slots as entries: more than half of a class's pairs
-// are free in a state below half filling), and the tables and workspace of the states.
+// Device memory of the tables, the FP64 workspace and the build, by the basis alone: row_ent and psi per
+// (row, pair), ent_row per slot (twice as many as entries: half of a class's pairs free in a state; 1.9 at
+// 3x9 Ne = 9, 2.2 at 5x5 Ne = 10), and the tables and workspace of the states.  The build counts slots and
+// states before it allocates, and asks again where they take more.
 int64_t pair_bytes(const momed_handle* h) {
     const int64_t e = h->n * pairs_per_row(h);
     return e * (4 + 16) + 2 * e * 4 + e * 8 / 3;
@@ -702,8 +703,9 @@ bool pair_possible(momed_handle* h) {
 }
 
 // Builds the tables (the caller has the index; lookups compare keys, so no validation of the
-// operator is needed).  Returns false, with nothing built, where the states have too few free pairs.
-bool build_pair_map(momed_handle* h) {
+// operator is needed).  Returns false, with nothing built, where the states have too few free pairs or
+// the tables do not fit after all.
+bool build_pair_map(momed_handle* h, double share) {
     PairMap& pm = h->hcache.pair;
     pm.release();
     const PairPlan& pl = h->pplan;
@@ -742,6 +744,11 @@ bool build_pair_map(momed_handle* h) {
     const int64_t pad = tiles * 32;
     const int64_t ids = std::accumulate(tc.begin(), tc.end(), (int64_t)0);
     if (pair_policy() != 1 && ((double)nent / (double)std::max<int64_t>(ids, 1) - 1.0) * pl.density < kMinHitsPerEntry) {
+        pm.declined = true;
+        return false;
+    }
+    const int64_t need = nent * (4 + 16 + 1) + slots * 4 + tiles * 16 + pad * 8;
+    if (need > pair_bytes(h) && !(share > 0.0 && fits_free(need, share))) {
         pm.declined = true;
         return false;
     }

@@ -337,7 +337,20 @@ void worker_loop(momed_server* S, int slot) {
                 if (hc_bytes > 0) {
                     try {
                         if (nu > 1 && hc_mode == 1) build_hit_records(h);
-                        else build_hit_cache(h, hc_mode);
+                        else build_hit_cache(h, hc_mode, 0.0);
+                        // what was held was an estimate, and where the pair tables are declined it was
+                        // that of other tables: from here on what the cache takes
+                        const int64_t takes = h->hcache.bytes;
+                        bool fits;
+                        {
+                            std::lock_guard<std::mutex> lk(S->mu);
+                            fits = S->used - hc_bytes + takes <= S->budget;
+                            if (fits) {
+                                S->used += takes - hc_bytes;
+                                hc_bytes = takes;
+                            }
+                        }
+                        if (!fits) unreserve();          // candidate map
                     } catch (const Error& e) {
                         if (e.code != MOMED_ENOMEM) throw;
                         unreserve();          // the device is shorter than the budget: candidate map

@@ -571,9 +571,10 @@ int momed_matvec(momed_handle* h, const void* x, void* y, int32_t precision, int
             ensure_index(h);
             if (!h->hcache.built && !h->hcache.pair.built) {
                 // a map applied again and again (an outer Krylov code): from the second call on a
-                // basis and operator, the pair tables, when they are admitted as the solvers' are
-                if (h->hcache.plain_calls > 0) ensure_plain_pair(h);
-                else ++h->hcache.plain_calls;
+                // basis and operator, the pair tables, when they are admitted as the solvers' are.
+                // Asked at calls 2, 3, 5, 9, ...: where they are not, asking took 0.1 to 14 ms a call
+                const int64_t c = h->hcache.plain_calls++;
+                if (c > 0 && (c & (c - 1)) == 0) ensure_plain_pair(h);
             }
             if (!h->hcache.built && !h->hcache.pair.built) ensure_ready(h);
         }

@@ -763,7 +763,6 @@ void ensure_plain_pair(momed_handle* h) {
     } catch (const Error& e) {
         if (e.code != MOMED_ENOMEM) throw;
         hc.pair.release();
-        hc.plain_calls = 0;
     }
 }
 

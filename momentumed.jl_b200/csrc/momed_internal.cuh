@@ -347,7 +347,7 @@ struct HitCache {
     int mode = 0;               // 1: full (pair tables, or target and term slot per hit), 2: term slots only
     bool records = false;       // the hit records are built (the block maps read them)
     PairMap pair;               // the single-vector map's tables, where the operator takes that form
-    int plain_calls = 0;        // momed_matvec calls on this basis and operator without a cache
+    int64_t plain_calls = 0;    // momed_matvec calls on this basis and operator without a cache
     int64_t nnz = 0, bytes = 0;
     double build_ms = 0.0;
     DevBuf<int64_t> row_ptr;

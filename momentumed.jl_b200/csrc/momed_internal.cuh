@@ -291,8 +291,9 @@ struct PairPlanView {
     const int4* cls;           // [nclass] {pairs P, offset in mask/coup, offset in V, 0}
     const uint64_t* mask;      // pair masks, class by class
     const uint32_t* coup;      // per pair: the pairs of its class it is coupled to (not itself)
-    const uint32_t* listed;    // the same with itself where the list has that term
     const int32_t* ptab;       // [64 * 64] class << 8 | slot of the pair {a < b}, -1: none
+    const int32_t* d1;         // [64] term slot of the orbital's one-body term, -1: none
+    const int32_t* d2;         // [64 * 64] term slot of the pair {a < b} with itself, -1: none
 };
 struct PairPlan {
     int state = -1;            // -1 not looked at, 0 the operator does not take the pair form, 1 ready
@@ -300,15 +301,12 @@ struct PairPlan {
     int64_t nv = 0;            // sum of P * P
     double density = 0.0;      // share of the off-diagonal couplings that the list has
     std::vector<int> P;        // pairs of each class
-    uint64_t has_d = 0;        // orbitals with a one-body term
     DevBuf<int4> cls;
     DevBuf<uint64_t> mask;
-    DevBuf<uint32_t> coup, listed;
-    DevBuf<int32_t> ptab, vslot, d1;   // vslot [nv] and d1 [64]: term slots of V and the one-body diagonal
-    DevBuf<double2> v64, d64;          // their values at u64 / u32
-    DevBuf<float2> v32, d32;
-    double u64 = 0.0, u32 = 0.0;
-    bool ok64 = false, ok32 = false;
+    DevBuf<uint32_t> coup;
+    DevBuf<int32_t> ptab, vslot, d1, d2;   // vslot [nv]: term slots of V
+    DevBuf<double2> v64;                   // V, at the u64 / u32 of the tables
+    DevBuf<float2> v32;
     PairPlanView view() const;
 };
 // Tables of the pair-factorised map for one basis (pairmap.cu).
@@ -329,9 +327,13 @@ struct PairMap {
     DevBuf<uint32_t> ent_row, row_ent;
     DevBuf<int4> work;
     DevBuf<double2> psi;       // workspace of a product, one value per entry (FP32 products use half of it)
+    DevBuf<double2> da, db;    // the rows' diagonal, A and B parts
+    bool ok_diag = false;
+    double u64 = 0.0, u32 = 0.0;       // the u of the plan's V
+    bool ok64 = false, ok32 = false;
     PairView view() const;
     void release() {
-        built = declined = false;
+        built = declined = ok_diag = ok64 = ok32 = false;
         n = entries = hits = bytes = 0;
         kmax = nwork = 0;
         tile.release();
@@ -339,6 +341,8 @@ struct PairMap {
         row_ent.release();
         work.release();
         psi.release();
+        da.release();
+        db.release();
     }
 };
 

@@ -8,8 +8,9 @@
 // taken in two steps through the states with two particles removed:
 //
 //   phi_q(s')  = sign(s', q) x[s' + q]           for every pair q of the class free in s'
-//   psi_p(s')  = sum_q V[p][q] phi_q(s')         (a dense P x P product per s', P = pairs of a class)
-//   y[s]       = sum over pairs p of s of sign(s - p, p) psi_p(s - p)  + one-body diagonal x[s]
+//   psi_p(s')  = sum_q V[p][q] phi_q(s')         (a dense P x P product per s', P = pairs of a class;
+//                                                 V[p][p] = 0: a pair with itself is of the diagonal)
+//   y[s]       = sum over pairs p of s of sign(s - p, p) psi_p(s - p)  + diagonal[s] x[s]
 //
 // The fermionic sign of a term factorises over its two pairs: popcount(s' & (pm_out ^ pm_in)) is
 // even exactly when those of its two masks agree.  A row has Ne (Ne - 1) / 2 pairs, so a map
@@ -266,27 +267,6 @@ template <typename R> __device__ __forceinline__ typename Cx<R>::T cx0() {
     return v;
 }
 
-// V[class][p][q] and the one-body diagonal per orbital at parameter u: A + u B of their term slots
-template <typename R>
-__global__ void k_pair_values(const int32_t* __restrict__ vslot, int64_t nv, const int32_t* __restrict__ d1,
-                              const typename Cx<R>::T* __restrict__ A, const typename Cx<R>::T* __restrict__ B, R u,
-                              typename Cx<R>::T* __restrict__ V, typename Cx<R>::T* __restrict__ D) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv + 64; i += (int64_t)gridDim.x * blockDim.x) {
-        const int t = i < nv ? __ldg(vslot + i) : __ldg(d1 + (i - nv));
-        typename Cx<R>::T a = cx0<R>();
-        if (t >= 0) {
-            a = A[t];
-            if (B) {
-                const typename Cx<R>::T b = B[t];
-                a.x += u * b.x;
-                a.y += u * b.y;
-            }
-        }
-        if (i < nv) V[i] = a;
-        else D[i - nv] = a;
-    }
-}
-
 // Four chains of FMAs per output; FP32 reads V two pairs at a time (16 bytes, as FP64 does one).
 // A value is finite when its parts' high bits without their signs (top: the larger) are below kInf.
 template <typename R> struct PairV;
@@ -309,6 +289,62 @@ template <> struct PairV<float> {
         return make_float2(__uint_as_float(__float_as_uint(x.x) ^ sign), __uint_as_float(__float_as_uint(x.y) ^ sign));
     }
 };
+// V[class][p][q] for the couplings of different pairs at parameter u: A + u B of their term slots
+template <typename R>
+__global__ void k_pair_values(const int32_t* __restrict__ vslot, int64_t nv, const typename Cx<R>::T* __restrict__ A,
+                              const typename Cx<R>::T* __restrict__ B, R u, typename Cx<R>::T* __restrict__ V) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (int64_t)gridDim.x * blockDim.x) {
+        const int t = __ldg(vslot + i);
+        typename Cx<R>::T a = cx0<R>();
+        if (t >= 0) {
+            a = A[t];
+            if (B) {
+                const typename Cx<R>::T b = B[t];
+                a.x += u * b.x;
+                a.y += u * b.y;
+            }
+        }
+        V[i] = a;
+    }
+}
+
+// Each row's diagonal, A and B parts in FP64: its one-body terms and its pairs with themselves, summed with
+// their rounding errors (Knuth's two-sum), as the diagonal is most of a row.  With V[p][p] in the products instead, c64 maps were 1.1 to 3.2 times as far from 64 bits as over
+// the hit records, which have the diagonal apart as well: 9.7e-8 against 3.6e-8 at 3x9 Ne = 9.
+__global__ void k_pair_diag(PairPlanView pp, const uint64_t* __restrict__ basis, int64_t n,
+                            const double2* __restrict__ A, const double2* __restrict__ B, double2* __restrict__ da,
+                            double2* __restrict__ db) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double2 a = make_double2(0.0, 0.0), b = a, ea = a, eb = a;
+        auto two = [](double& s, double& e, double v) {
+            const double t = s + v, z = t - s;
+            e += (s - (t - z)) + (v - z);
+            s = t;
+        };
+        auto add = [&](int t) {
+            if (t < 0) return;
+            const double2 v = __ldg(A + t);
+            two(a.x, ea.x, v.x);
+            two(a.y, ea.y, v.y);
+            if (B) {
+                const double2 w = __ldg(B + t);
+                two(b.x, eb.x, w.x);
+                two(b.y, eb.y, w.y);
+            }
+        };
+        for (uint64_t h = __ldg(basis + i); h; h &= h - 1ull) {
+            const int lo = __ffsll((long long)h) - 1;
+            add(__ldg(pp.d1 + lo));
+            for (uint64_t g = h & (h - 1ull); g; g &= g - 1ull)
+                add(__ldg(pp.d2 + lo * 64 + __ffsll((long long)g) - 1));
+        }
+        // (an infinite sum has no error to add)
+        auto join = [](double s, double e) { return isfinite(e) ? s + e : s; };
+        da[i] = make_double2(join(a.x, ea.x), join(a.y, ea.y));
+        if (B) db[i] = make_double2(join(b.x, eb.x), join(b.y, eb.y));
+    }
+}
+
 // row length of V in shared memory: even for FP32, whose loads take two values
 template <typename R> __host__ __device__ constexpr int pair_ld(int pm) { return std::is_same<R, float>::value ? (pm + 1) / 2 * 2 : pm; }
 
@@ -410,12 +446,12 @@ k_pair_ids(PairView pv, PairPlanView pp, const typename Cx<R>::T* __restrict__ V
 // 20.4).  Tests in k_pair_ids cost 1 to 15% of the map, on its values, its products or once per tile.
 template <typename R>
 __device__ __noinline__ typename Cx<R>::T pair_row_apart(const PairPlanView& pp, const uint64_t* basis, int64_t n,
-                                                         int64_t row, const typename Cx<R>::T* V,
-                                                         const typename Cx<R>::T* Ds, uint64_t has_d,
+                                                         int64_t row, const typename Cx<R>::T* V, double2 d,
                                                          const typename Cx<R>::T* x) {
     using C2 = typename Cx<R>::T;
     const uint64_t s = basis[row];
     C2 acc = cx0<R>();
+    bool diag = false;                                        // the row has a diagonal term
     auto add = [&](C2 c, int64_t j, bool neg) {
         const C2 v = x[j];
         const R pr = c.x * v.x - c.y * v.y, pi = c.x * v.y + c.y * v.x;
@@ -425,16 +461,17 @@ __device__ __noinline__ typename Cx<R>::T pair_row_apart(const PairPlanView& pp,
 #pragma unroll 1
     for (uint64_t h = s; h; h &= h - 1ull) {
         const int lo = __ffsll((long long)h) - 1;
-        if ((has_d >> lo) & 1ull) add(Ds[lo], row, false);
+        diag |= pp.d1[lo] >= 0;
 #pragma unroll 1
         for (uint64_t g = h & (h - 1ull); g; g &= g - 1ull) {
             const int hi = __ffsll((long long)g) - 1, cs = pp.ptab[lo * 64 + hi];
             if (cs < 0) continue;
+            diag |= pp.d2[lo * 64 + hi] >= 0;
             const int4 cl = pp.cls[cs >> 8];
             const int p = cs & 255;
             const uint64_t mp = (1ull << lo) | (1ull << hi), rest = s & ~mp;
 #pragma unroll 1
-            for (uint32_t m = pp.listed[cl.y + p]; m; m &= m - 1u) {
+            for (uint32_t m = pp.coup[cl.y + p]; m; m &= m - 1u) {
                 const int q = __ffs((int)m) - 1;
                 const uint64_t mq = pp.mask[cl.y + q], t = rest | mq;
                 if (rest & mq) continue;
@@ -449,26 +486,41 @@ __device__ __noinline__ typename Cx<R>::T pair_row_apart(const PairPlanView& pp,
             }
         }
     }
+    if (diag) {
+        C2 c;
+        c.x = (R)d.x;
+        c.y = (R)d.y;
+        add(c, row, false);
+    }
     return acc;
 }
 
-// y[row] = sum of the psi of the row's pairs + one-body diagonal x[row] (has_d: the orbitals with a one-body
-// term): a lane per row, G warps share the pairs of 32 rows (sums combined in a fixed order).
+// y[row] = sum of the psi of the row's pairs + diagonal x[row]: a lane per row, G warps share the pairs of 32
+// rows (sums combined in a fixed order, in FP64 for FP32 values, too: 471 us against 445 in FP32 on two-
+// component 4x6, where the error over the hit records' falls from 1.02 to 0.997).
 template <typename R>
-__global__ void __launch_bounds__(kPT)
+__global__ void __launch_bounds__(kPT, std::is_same<R, double>::value ? 4 : 5)    // no spills from here up
 k_pair_rows(PairView pv, PairPlanView pp, const uint64_t* __restrict__ basis, const typename Cx<R>::T* __restrict__ V,
-            const typename Cx<R>::T* __restrict__ D, uint64_t has_d, const typename Cx<R>::T* __restrict__ psi,
+            const double2* __restrict__ da, const double2* __restrict__ db, double u,
+            const typename Cx<R>::T* __restrict__ psi,
             const typename Cx<R>::T* __restrict__ x, typename Cx<R>::T* __restrict__ y, int G) {
     using C2 = typename Cx<R>::T;
-    __shared__ C2 Ds[64];
-    __shared__ C2 part[kPT];
-    if (threadIdx.x < 64) Ds[threadIdx.x] = D[threadIdx.x];
-    __syncthreads();
+    __shared__ double2 part[kPT];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = wid % G;
     const int64_t row = ((int64_t)blockIdx.x * (kPT / 32 / G) + wid / G) * 32 + lane;
-    C2 acc = cx0<R>();
+    double2 acc = make_double2(0.0, 0.0), d = acc;
+    C2 xv = cx0<R>();
     if (row < pv.n) {
+        if (g == 0) {
+            d = __ldg(da + row);
+            xv = __ldg(x + row);
+            if (db) {
+                const double2 b = __ldg(db + row);
+                d.x += u * b.x;
+                d.y += u * b.y;
+            }
+        }
         const uint32_t* re = pv.row_ent + row;
         int k = g;
         for (; k + 5 * G < pv.kmax; k += 6 * G) {
@@ -479,7 +531,9 @@ k_pair_rows(PairView pv, PairPlanView pp, const uint64_t* __restrict__ basis, co
 #pragma unroll
             for (int i = 0; i < 6; ++i) v[i] = e[i] != kNoEntry ? __ldg(psi + e[i]) : cx0<R>();
 #pragma unroll
-            for (int i = 0; i < 6; ++i) { acc.x += v[i].x; acc.y += v[i].y; }
+            for (int i = 0; i < 3; ++i) { v[i].x += v[i + 3].x; v[i].y += v[i + 3].y; }
+            acc.x += v[0].x + (v[1].x + v[2].x);
+            acc.y += v[0].y + (v[1].y + v[2].y);
         }
         for (; k < pv.kmax; k += G) {
             const uint32_t e = __ldg(re + (int64_t)k * pv.n);
@@ -489,32 +543,24 @@ k_pair_rows(PairView pv, PairPlanView pp, const uint64_t* __restrict__ basis, co
                 acc.y += v.y;
             }
         }
-        if (g == 0) {
-            C2 d = cx0<R>();
-            for (uint64_t s = __ldg(basis + row); s; s &= s - 1ull) {
-                const C2 o = Ds[__ffsll((long long)s) - 1];
-                d.x += o.x;
-                d.y += o.y;
-            }
-            const C2 xv = __ldg(x + row);
-            acc.x += d.x * xv.x - d.y * xv.y;
-            acc.y += d.x * xv.y + d.y * xv.x;
-        }
     }
     if (G > 1) {
         part[threadIdx.x] = acc;
         __syncthreads();
         if (g == 0) {
             for (int i = 1; i < G; ++i) {
-                const C2 v = part[threadIdx.x + 32 * i];
+                const double2 v = part[threadIdx.x + 32 * i];
                 acc.x += v.x;
                 acc.y += v.y;
             }
         }
     }
     if (g == 0 && row < pv.n) {
-        if (PairV<R>::top(acc) >= PairV<R>::kInf) acc = pair_row_apart<R>(pp, basis, pv.n, row, V, Ds, has_d, x);
-        y[row] = acc;
+        C2 o;                                     // the diagonal is most of y: joined and rounded once
+        o.x = (R)fma(d.x, (double)xv.x, fma(-d.y, (double)xv.y, acc.x));
+        o.y = (R)fma(d.x, (double)xv.y, fma(d.y, (double)xv.x, acc.y));
+        if (PairV<R>::top(o) >= PairV<R>::kInf) o = pair_row_apart<R>(pp, basis, pv.n, row, V, d, x);
+        y[row] = o;
     }
 }
 
@@ -541,8 +587,9 @@ PairPlanView PairPlan::view() const {
     v.cls = cls.p;
     v.mask = mask.p;
     v.coup = coup.p;
-    v.listed = listed.p;
     v.ptab = ptab.p;
+    v.d1 = d1.p;
+    v.d2 = d2.p;
     return v;
 }
 
@@ -620,8 +667,8 @@ bool pair_plan(momed_handle* h) {
         pmax = std::max(pmax, P[c]);
     }
     std::vector<uint64_t> mask(np);
-    std::vector<uint32_t> coup(np, 0u), listed(np, 0u);
-    std::vector<int32_t> ptab(64 * 64, -1), vslot(voff, -1);
+    std::vector<uint32_t> coup(np, 0u);
+    std::vector<int32_t> ptab(64 * 64, -1), d2(64 * 64, -1), vslot(voff, -1);
     for (int i = 0; i < np; ++i) {
         mask[cls[cls_of[i]].y + slot_of[i]] = pairs[i];
         const int lo = __builtin_ctzll(pairs[i]), hi = 63 - __builtin_clzll(pairs[i]);
@@ -632,9 +679,10 @@ bool pair_plan(momed_handle* h) {
         if (__builtin_popcountll(tout[t]) == 2) {
             const int o = at(tout[t]), i = at(tin[t]);
             const int4 c = cls[cls_of[o]];
-            vslot[c.z + slot_of[o] * c.x + slot_of[i]] = (int32_t)t;
-            listed[c.y + slot_of[o]] |= 1u << slot_of[i];
-            if (o != i) {
+            if (o == i) {
+                d2[__builtin_ctzll(pairs[o]) * 64 + 63 - __builtin_clzll(pairs[o])] = (int32_t)t;
+            } else {
+                vslot[c.z + slot_of[o] * c.x + slot_of[i]] = (int32_t)t;
                 coup[c.y + slot_of[o]] |= 1u << slot_of[i];
                 ++ncoup;
             }
@@ -643,20 +691,16 @@ bool pair_plan(momed_handle* h) {
     upload(pl.cls, cls, st);
     upload(pl.mask, mask, st);
     upload(pl.coup, coup, st);
-    upload(pl.listed, listed, st);
     upload(pl.ptab, ptab, st);
     upload(pl.vslot, vslot, st);
     upload(pl.d1, d1, st);
+    upload(pl.d2, d2, st);
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));
     pl.P = P;
-    pl.has_d = 0;
-    for (int o = 0; o < 64; ++o)
-        if (d1[o] >= 0) pl.has_d |= 1ull << o;
     pl.nclass = nc;
     pl.pmax = pmax;
     pl.nv = voff;
     pl.density = voff > np ? (double)ncoup / (double)(voff - np) : 0.0;
-    pl.ok64 = pl.ok32 = false;
     pl.state = 1;
     return true;
 }
@@ -669,11 +713,11 @@ static int64_t pairs_per_row(const momed_handle* h) {
 
 // Device memory of the tables, the FP64 workspace and the build, by the basis alone: row_ent and psi per
 // (row, pair), ent_row per slot (twice as many as entries: half of a class's pairs free in a state; 1.9 at
-// 3x9 Ne = 9, 2.2 at 5x5 Ne = 10), and the tables and workspace of the states.  The build counts slots and
+// 3x9 Ne = 9, 2.2 at 5x5 Ne = 10), the tables and workspace of the states, and the rows' diagonals.  The build counts slots and
 // states before it allocates, and asks again where they take more.
 int64_t pair_bytes(const momed_handle* h) {
     const int64_t e = h->n * pairs_per_row(h);
-    return e * (4 + 16) + 2 * e * 4 + e * 8 / 3;
+    return e * (4 + 16) + 2 * e * 4 + e * 8 / 3 + h->n * 32;
 }
 
 // MOMED_PAIRMAP=0: never, =1: whatever the size and density
@@ -700,6 +744,19 @@ bool pair_possible(momed_handle* h) {
     if (h->n <= 0 || h->n >= (int64_t)0x7fffffff || k < 1 || k > 2016) return false;
     if (h->n * k >= (int64_t)kNoEntry) return false;      // entries are 32-bit, and so is a row block's item count
     return pair_plan(h);
+}
+
+// the rows' diagonals from the term amplitudes
+static void pair_diag(momed_handle* h) {
+    PairMap& pm = h->hcache.pair;
+    const OpView ov = h->op.view();
+    pm.da.resize(pm.n);
+    if (ov.t_ampb) pm.db.resize(pm.n);
+    k_pair_diag<<<(unsigned)std::min<int64_t>((pm.n + 255) / 256, 1184), 256, 0, h->stream>>>(
+        h->pplan.view(), h->basis.p, pm.n, ov.t_amp, ov.t_ampb, pm.da.p, pm.db.p);
+    MOMED_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    pm.ok_diag = true;
 }
 
 // Builds the tables (the caller has the index; lookups compare keys, so no validation of the
@@ -747,7 +804,7 @@ bool build_pair_map(momed_handle* h, double share) {
         pm.declined = true;
         return false;
     }
-    const int64_t need = nent * (4 + 16 + 1) + slots * 4 + tiles * 16 + pad * 8;
+    const int64_t need = nent * (4 + 16 + 1) + slots * 4 + tiles * 16 + pad * 8 + n * 32;
     if (need > pair_bytes(h) && !(share > 0.0 && fits_free(need, share))) {
         pm.declined = true;
         return false;
@@ -792,12 +849,15 @@ bool build_pair_map(momed_handle* h, double share) {
         pm.release();
         throw Error{MOMED_EINVAL, "pair map: table passes disagree"};
     }
-    pm.n = n;
     pm.kmax = kmax;
     pm.entries = (int64_t)th[0];
-    pm.psi.resize(std::max<int64_t>(pm.entries, 1));   // here, so that the first product does not wait for it
+    // here, so that the first product does not wait for them
+    pm.psi.resize(std::max<int64_t>(pm.entries, 1));
+    pm.n = n;
+    pair_diag(h);
     pm.hits = (int64_t)th[1];
-    pm.bytes = (int64_t)(pm.work.bytes() + pm.tile.bytes() + pm.ent_row.bytes() + pm.row_ent.bytes() + pm.psi.bytes());
+    pm.bytes = (int64_t)(pm.work.bytes() + pm.tile.bytes() + pm.ent_row.bytes() + pm.row_ent.bytes() + pm.psi.bytes() +
+                         pm.da.bytes() + pm.db.bytes());
     pm.built = true;
     return true;
 }
@@ -807,17 +867,15 @@ namespace {
 template <typename R> struct PairSlot;
 template <> struct PairSlot<double> {
     static DevBuf<double2>& v(PairPlan& p) { return p.v64; }
-    static DevBuf<double2>& d(PairPlan& p) { return p.d64; }
-    static double& u(PairPlan& p) { return p.u64; }
-    static bool& ok(PairPlan& p) { return p.ok64; }
+    static double& u(PairMap& m) { return m.u64; }
+    static bool& ok(PairMap& m) { return m.ok64; }
     static const double2* a(const OpView& o) { return o.t_amp; }
     static const double2* b(const OpView& o) { return o.t_ampb; }
 };
 template <> struct PairSlot<float> {
     static DevBuf<float2>& v(PairPlan& p) { return p.v32; }
-    static DevBuf<float2>& d(PairPlan& p) { return p.d32; }
-    static double& u(PairPlan& p) { return p.u32; }
-    static bool& ok(PairPlan& p) { return p.ok32; }
+    static double& u(PairMap& m) { return m.u32; }
+    static bool& ok(PairMap& m) { return m.ok32; }
     static const float2* a(const OpView& o) { return o.t_amp32; }
     static const float2* b(const OpView& o) { return o.t_ampb32; }
 };
@@ -838,16 +896,16 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
     if (pm.n <= 0) return;
     const OpView ov = h->op.view();
     auto& V = S::v(pl);
-    auto& D = S::d(pl);
     C2* psi = reinterpret_cast<C2*>(pm.psi.p);
-    if (!S::ok(pl) || (ov.t_ampb && S::u(pl) != u)) {         // formed again for another u or new amplitudes
+    if (!S::ok(pm) || (ov.t_ampb && S::u(pm) != u)) {         // formed again for another u or new amplitudes
         V.resize(std::max<int64_t>(pl.nv, 1));
-        D.resize(64);
-        k_pair_values<R><<<(unsigned)std::min<int64_t>((pl.nv + 64 + 255) / 256, 1184), 256, 0, st>>>(
-            pl.vslot.p, pl.nv, pl.d1.p, S::a(ov), S::b(ov), (R)u, V.p, D.p);
+        k_pair_values<R><<<(unsigned)std::min<int64_t>((pl.nv + 255) / 256, 1184), 256, 0, st>>>(
+            pl.vslot.p, pl.nv, S::a(ov), S::b(ov), (R)u, V.p);
+        MOMED_CUDA_TRY(cudaGetLastError());
         note_launches(1);
-        S::u(pl) = u;
-        S::ok(pl) = true;
+        if (!pm.ok_diag) pair_diag(h);                        // new amplitudes without a rebuild
+        S::u(pm) = u;
+        S::ok(pm) = true;
     }
     if (pm.nwork > 0) {
         // instantiated pair counts: every even one to 16 and the odd ones that meshes of 21 to 30
@@ -876,8 +934,8 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
     int G = 1;
     while (G < 8 && rw * G < want) G *= 2;
     const int per = kPT / 32 / G;
-    k_pair_rows<R><<<(unsigned)((rw + per - 1) / per), kPT, 0, st>>>(pm.view(), pl.view(), h->basis.p, V.p, D.p, pl.has_d, psi, x,
-                                                                     y, G);
+    k_pair_rows<R><<<(unsigned)((rw + per - 1) / per), kPT, 0, st>>>(pm.view(), pl.view(), h->basis.p, V.p, pm.da.p, ov.t_ampb ? pm.db.p : nullptr,
+                                                                     u, psi, x, y, G);
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
 }

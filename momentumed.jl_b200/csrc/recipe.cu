@@ -232,7 +232,7 @@ void set_kshift(momed_handle* h, const double* kshift) {
     }
     MOMED_CUDA_TRY(cudaStreamSynchronize(st));   // sh is read by the async copy
     h->sparse.release();                          // its values were built from the old amplitudes
-    h->pplan.ok64 = h->pplan.ok32 = false;        // the pair form's values come from the term amplitudes
+    h->hcache.pair.ok64 = h->hcache.pair.ok32 = h->hcache.pair.ok_diag = false;   // formed from the term amplitudes
     if (h->op.has_b) h->hcache.release();         // its runs are sorted by which parts are non-zero
 }
 

@@ -585,9 +585,13 @@ struct BlockLanczos {
         // and one flagged right-hand side makes the whole block repeat the pass.  Measured on B200:
         // with FP64 bases, or few wanted pairs (nev <= m/5), 0.1 runs the same maps and gives the same
         // eigenvalues as 1/2 (3x9, 32 U0, nev 4: 16% faster; 0.01 the same).  FP32 bases with more
-        // wanted pairs take 0.2: over 3x8, 3x9 and 4x6 sectors, 1 and 8 right-hand sides, nev 7 to 20
-        // in m 24 to 64 and three seeds the maps are those of 1/2 (within a restart cycle either way)
-        // and the time 2 to 25% less: 3x9, nev 7 in m 30 41.3 -> 37.3 ms alone, 191 -> 162 ms for 8.
+        // wanted pairs take 0.2: over 448 mixed solves (ten operators, 3x8, 3x9, 4x6 and two-component
+        // 4x4 sectors, two to four seeds, 1 and 8 right-hand sides, nev 7 to 20 in m 30 to 64) 13% less
+        // time than 1/2 in the mean, 0.3 12% and 0.4 9%.  Any change of rounding moves a solve's maps by
+        // a refinement cycle, or in and out of the FP64 lockstep solve that follows the last one: single
+        // solves took 0.44 to 1.76 times 1/2's time.  But no rule needs it more often (38 / 33 / 37 / 36
+        // of the 448 at 1/2, 0.4, 0.3, 0.2), and the maps are 3.6 / 3.2 / 3.4 / 3.2% above the fewest of
+        // the four in the mean.
         dgks = (std::is_same<VT, float2>::value && 5 * nev > m) ? 0.2 : 0.1;
         // graphs captured by an earlier run of this object carry that run's dgks: capture anew
         for (auto& g : graphs) cudaGraphExecDestroy(g.exec);

@@ -908,8 +908,9 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
         S::ok(pm) = true;
     }
     if (pm.nwork > 0) {
-        // instantiated pair counts: every even one to 16 and the odd ones that meshes of 21 to 30
-        // orbitals have (13, 15), then steps of 4; a class pads to the next
+        // instantiated pair counts: every even one to 16 and of the odd ones 13 and 15 (meshes of 26, 27
+        // and 30, 31 orbitals, 3x9 and 3x10 among them), then steps of 4; a class pads to the next (11 pairs,
+        // of 22 and 23 orbitals, to 12)
         switch (pl.pmax <= 4 ? 4 : pl.pmax <= 16 ? (pl.pmax == 13 || pl.pmax == 15 ? pl.pmax : (pl.pmax + 1) / 2 * 2)
                                                  : (pl.pmax + 3) / 4 * 4) {
             case 4: ids_launch<R, 4>(pm, pl, V.p, x, psi, st); break;

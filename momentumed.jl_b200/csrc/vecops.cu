@@ -380,7 +380,12 @@ void vec_random(VT* v, int64_t N, uint64_t seed, cudaStream_t st) {
     MOMED_CUDA_TRY(cudaGetLastError());
     note_launches(1);
 }
-int vec_combine_group(int nout) { return nout >= 24 ? 8 : 4; }
+// Groups of 4 as long as every group has a warp of the block to itself (32 outputs), then of 8, which
+// halve the rounds.  4 / 8, in us: 174k states 82 / 110 with 24 kept vectors, 132 / 152 with 32, 175 / 173
+// with 33, 277 / 200 with 43; 1.0M states 429 / 597, 693 / 831, 891 / 943, 1052 / 1021 (38); 31k states
+// 23 / 24, 31 / 30 (31), 46 / 34 (33), 63 / 48 (48); FP32 vectors, 174k states, 77 / 100 (24), 108 / 132
+// (32), 164 / 160 (33).
+int vec_combine_group(int nout) { return nout > 4 * (kVecThreads / 32) ? 8 : 4; }
 
 std::vector<double> vec_pack_coefs(const std::vector<double>& U, int m, int nout) {
     const int oc = vec_combine_group(nout);

@@ -442,8 +442,8 @@ k_pair_ids(PairView pv, PairPlanView pp, const typename Cx<R>::T* __restrict__ V
 // and pairs that a state lacks (phi = 0) along, which add nothing to finite values but spread an infinity
 // or a NaN of x or V over the class; here it stays with the rows that the list connects to it.  Rare, so
 // targets are searched in the sorted basis, and a test per row is all that the usual rows pay (48 registers
-// instead of 32: 205 -> 200 us for c128 on 1.0M states, 16.6 -> 17.6 for c64 on 174k; held to 32: 224 and
-// 20.4).  Tests in k_pair_ids cost 1 to 15% of the map, on its values, its products or once per tile.
+// instead of 32, before the rows' sums were FP64 throughout: 205 -> 200 us for c128 on 1.0M states, 16.6 ->
+// 17.6 for c64 on 174k; held to 32: 224 and 20.4).  Tests in k_pair_ids cost 1 to 15% of the map, on its values, its products or once per tile.
 template <typename R>
 __device__ __noinline__ typename Cx<R>::T pair_row_apart(const PairPlanView& pp, const uint64_t* basis, int64_t n,
                                                          int64_t row, const typename Cx<R>::T* V, double2 d,

@@ -509,25 +509,14 @@ k_pair_rows(PairView pv, PairPlanView pp, const uint64_t* __restrict__ basis, co
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = wid % G;
     const int64_t row = ((int64_t)blockIdx.x * (kPT / 32 / G) + wid / G) * 32 + lane;
-    double2 acc = make_double2(0.0, 0.0), d = acc;
-    C2 xv = cx0<R>();
+    double2 acc = make_double2(0.0, 0.0);
     if (row < pv.n) {
-        if (g == 0) {
-            d = __ldg(da + row);
-            xv = __ldg(x + row);
-            if (db) {
-                const double2 b = __ldg(db + row);
-                d.x += u * b.x;
-                d.y += u * b.y;
-            }
-        }
         const uint32_t* re = pv.row_ent + row;
-        int k = g;
-        for (; k + 5 * G < pv.kmax; k += 6 * G) {
+        for (int k = g; k < pv.kmax; k += 6 * G) {
             uint32_t e[6];
             C2 v[6];
 #pragma unroll
-            for (int i = 0; i < 6; ++i) e[i] = ld_stream(re + (int64_t)(k + i * G) * pv.n);
+            for (int i = 0; i < 6; ++i) e[i] = k + i * G < pv.kmax ? ld_stream(re + (int64_t)(k + i * G) * pv.n) : kNoEntry;
 #pragma unroll
             for (int i = 0; i < 6; ++i) v[i] = e[i] != kNoEntry ? __ldg(psi + e[i]) : cx0<R>();
 #pragma unroll
@@ -535,13 +524,16 @@ k_pair_rows(PairView pv, PairPlanView pp, const uint64_t* __restrict__ basis, co
             acc.x += v[0].x + (v[1].x + v[2].x);
             acc.y += v[0].y + (v[1].y + v[2].y);
         }
-        for (; k < pv.kmax; k += G) {
-            const uint32_t e = __ldg(re + (int64_t)k * pv.n);
-            if (e != kNoEntry) {
-                const C2 v = __ldg(psi + e);
-                acc.x += v.x;
-                acc.y += v.y;
-            }
+    }
+    double2 d = make_double2(0.0, 0.0);
+    C2 xv = cx0<R>();
+    if (g == 0 && row < pv.n) {
+        d = __ldg(da + row);
+        xv = __ldg(x + row);
+        if (db) {
+            const double2 b = __ldg(db + row);
+            d.x += u * b.x;
+            d.y += u * b.y;
         }
     }
     if (G > 1) {
@@ -930,8 +922,12 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
         MOMED_CUDA_TRY(cudaGetLastError());
         note_launches(1);
     }
-    // warps per 32 rows: enough of them to cover the gathers' latency on small sectors
-    const int64_t rw = (pm.n + 31) / 32, want = (int64_t)pair_sms() * 64;
+    // Warps per 32 rows: enough of them to cover the gathers' latency on small sectors, 16 an SM; more
+    // only share the row's sums.  A map with 1 / 2 / 4 of them, in us: c128 30.4 / 28.4 / 30.2 on 43k
+    // states (1.4k warps of rows), 98.5 / 100.4 / 104 on 131k, 107.9 / 105.9 / 109.9 on 174k, 146.4 / 148.7 /
+    // 152.8 on 247k; c64 25.4 / 24.4 / 24.3, 68.8 / 70.7 / 70.6, 68.8 / 71.3 / 75.0, 99.6 / 99.6 / 104.8.
+    // (64 an SM, for a kernel of 32 registers, cost this one up to 17%: 115.1 on 131k states, c128.)
+    const int64_t rw = (pm.n + 31) / 32, want = (int64_t)pair_sms() * 16;
     int G = 1;
     while (G < 8 && rw * G < want) G *= 2;
     const int per = kPT / 32 / G;

@@ -720,13 +720,13 @@ static int pair_policy() {
 
 // Below 2^20 entries the two launches of a product lose what the gathers save: on the B200, FP64 /
 // FP32, against the hit records, 30.6k states x 28 pairs (858k entries) 26.7 / 23.1 us against 28-29
-// / 21.2, 7.1k x 15 (106k) 17.5 / 16.9 against 12.1 / 10.6, but 43k x 28 (1.2M) 32.2 / 27.8 against
+// / 21.2, 7.1k x 15 (106k) 17.5 / 16.9 against 12.1 / 10.6, but 43k x 28 (1.2M) 28.4 / 25.3 against
 // 40.3 / 28.9.
 constexpr int64_t kMinEntries = 1 << 20;
 // Hits an entry has to stand for: the records visit them one by one, the pair form takes P products
 // instead, so a nearly half-filled lattice (few free pairs per state) gains nothing.  3.4 hits per
-// entry (4x6 Ne = 11) ran 109 us against 98, 4.4 (5x5 Ne = 10) 102 against 126, 4.7 (3x9 Ne = 11)
-// 437 against 546, 6.0 (3x9 Ne = 9) 105 against 180, 6.5 (4x7 Ne = 9) 147 against 261.
+// entry (4x6 Ne = 11) ran 109 us against 98, 4.4 (5x5 Ne = 10) 98 against 126, 4.7 (3x9 Ne = 11)
+// 437 against 546, 6.0 (3x9 Ne = 9) 108 against 180, 6.5 (4x7 Ne = 9) 147 against 261.
 constexpr double kMinHitsPerEntry = 4.0;
 
 bool pair_possible(momed_handle* h) {

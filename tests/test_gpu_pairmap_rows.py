@@ -1,5 +1,5 @@
 """Second half of the product over the pair tables (csrc/pairmap.cu): 8, 4, 2 and 1 warps share 32 rows by the
-sector's size, each summing its pairs six at a time with a remainder.
+sector's size, each summing its pairs six (c128) or twelve (c64) at a time with a remainder.
 
 Bars against the map over the hit records: complex128 1e-13, complex64 2e-6 relative (those of
 test_gpu_pairmap.py).

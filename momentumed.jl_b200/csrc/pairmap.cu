@@ -931,7 +931,7 @@ void pair_apply(momed_handle* h, const typename Cx<R>::T* x, typename Cx<R>::T* 
     // Warps per 32 rows: enough of them to cover the gathers' latency on small sectors, 16 an SM; more
     // only share the row's sums.  A map with 1 / 2 / 4 of them, in us: c128 30.4 / 28.4 / 30.2 on 43k
     // states (1.4k warps of rows), 98.5 / 100.4 / 104 on 131k, 107.9 / 105.9 / 109.9 on 174k, 146.4 / 148.7 /
-    // 152.8 on 247k; c64 25.4 / 24.4 / 24.3, 68.8 / 70.7 / 70.6, 68.8 / 71.3 / 75.0, 99.6 / 99.6 / 104.8.
+    // 152.8 on 247k; c64 with 1 / 2 24.3 / 24.4, 66.8 / 68.9, 69.3 / 71.1, 97.2 / 99.2.
     // (64 an SM, for a kernel of 32 registers, cost this one up to 17%: 115.1 on 131k states, c128.)
     const int64_t rw = (pm.n + 31) / 32, want = (int64_t)pair_sms() * 16;
     int G = 1;
